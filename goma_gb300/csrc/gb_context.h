@@ -28,7 +28,7 @@ struct Context {
   int path = 0;
   int tc_grid = 0;     // persistent grid of the DMMA kernels
   // ILU triangular solves: 0 sync-free sweeps, 1 level-scheduled graph,
-  // 2 automatic (the graph for short level schedules)
+  // 2 automatic (the sync-free sweeps)
   int trsv = 2;
   // host-injected fault of the sync-free sweeps (gb_set_sweep_fault)
   long long sweep_spin_limit = 0;  // polls per wait; <= 0: the default

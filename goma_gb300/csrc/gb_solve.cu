@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gb_context.h"
+#include "gb_publish.cuh"
 #include "gb_solve.h"
 
 namespace gb {
@@ -42,23 +43,6 @@ __device__ __forceinline__ float warp_sumf(float v) {
   return v;
 }
 
-// Arithmetic type of the vector kernels: FP64 data is combined in FP64, FP32
-// data in FP32.  On GB300 FP64 arithmetic runs at 1/64 of the FP32 rate, so
-// an FP32 kernel that widened its operands to FP64 would be bound by the
-// FP64 pipe instead of HBM; the FP32 inner solve gets its accuracy from the
-// FP64 refinement around it.
-template <class T>
-struct AccT {
-  using type = double;
-};
-template <>
-struct AccT<float> {
-  using type = float;
-};
-template <class T>
-using acc_t = typename AccT<T>::type;
-__device__ __forceinline__ double fmx(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fmx(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double wsum(double v) { return warp_sum(v); }
 __device__ __forceinline__ float wsum(float v) { return warp_sumf(v); }
 
@@ -610,64 +594,27 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Sync-free triangular solves: one launch per sweep, one CTA per node at a
-// time.  The nodes are numbered ("tickets") in the order of their
-// dependency levels (the level schedule of the sweep: all of level 0, then
-// level 1, ...; independent problems in one matrix interleave), and CTA b of
-// a G-CTA grid takes tickets b, b + G, b + 2G, ... in turn -- no atomic, and
-// a CTA reads its next node's ticket entry while it works on the current
-// one.  Per ticket a table holds the node's first unknown, unknown count and
-// block-inverse offset; per row one holds its off-node segment; the factor
-// values and column indices of the segments are stored in the sweep's own
-// (level-sorted) order, so a CTA reaches its rows' data in two dependent
-// loads.  A sweep
-// reads its right-hand side from one vector and writes its solution into
-// another that was filled beforehand with an "unpublished" sentinel (a
-// signalling NaN: arithmetic never produces one, so every computed value,
-// NaNs included, differs from it).  A node needs exactly the solution
-// values its rows reference, so it polls those values themselves until none
-// is the sentinel -- no per-node flag, no fence: each value is published by
-// one single-copy-atomic store.  The node is solved in two stages:
-//   A  all warps: for every row of the node, the right-hand side less the
-//      dot product with the solution values of OTHER nodes (the long part of
-//      the row, rows spread over the warps; each lane keeps its polled values
-//      in registers and adds them in a fixed order, so the result does not
-//      depend on arrival order);
-//   B  warp 0, lane r for row r: row r of the node's precomputed diagonal-
-//      block inverse (block_inverse_kernel, in shared memory) times those
-//      values -- independent products, no chain of substitution steps.
-// A warp loads its first row's factor values and column indices, and the
-// CTA the block inverse, before it polls, so only the gather of the
-// solution values stays on the critical path.  A node depends
-// only on nodes of lower levels, which hold earlier tickets; every CTA of the
-// grid is resident and takes its tickets in increasing order, so the lowest
-// unfinished ticket always has all its dependencies published and is held
-// by a CTA that is working on it: the sweep makes progress.  Every wait is bounded: past spin_limit polls the
-// CTA records an error, computes and publishes anyway (so no other CTA can
-// wait forever), every later wait of the sweep stops within 1024 polls, and
-// the host reports the failure after the sweep.  A legitimate wait lasts
-// microseconds; the default limit (kSpinLimit) is ~0.3 s.
+// Triangular solves: the sync-free sweeps by lines of nodes (gb_sweep.cu), or
+// one launch per dependency level (trsv_level_cta_kernel).
 //
-// Row structure used by the split: a node's unknowns are contiguous and
+// A sync-free sweep reads its right-hand side from one vector and writes its
+// solution into another that was filled beforehand with an "unpublished"
+// sentinel (a signalling NaN: arithmetic never produces one, so every
+// computed value, NaNs included, differs from it).  Whoever needs a solution
+// value polls the value itself -- no flag, no fence: each is published by one
+// single-copy-atomic store.  A legitimate wait lasts microseconds; the default
+// limit of a wait (kSpinLimit) is ~0.3 s.
+//
+// Row structure used here: a node's unknowns are contiguous and
 // every row of the node holds every own-node column except the energy row,
 // which lacks the pressure columns (they come last).  So in row i (local
 // index r) the own-node columns below the diagonal are the r entries just
 // before it, and those above are the next nr-1-r entries (nvn-1-r for the
 // energy row).
 static constexpr long long kSpinLimit = 1LL << 22;
-// row entries per lane loaded before the wait: 320 a row in FP32, 256 in
-// FP64 (where ten would spill at the 64 registers of four CTAs per SM)
-template <class T> constexpr int kPrefetchOf = sizeof(T) == 4 ? 10 : 8;
 static constexpr int kTrsvThreads = 256;
 
 struct TrsvArgs {
-  // the sync-free sweep's own tables, set per sweep: per ticket the node's
-  // (unknown count << 32 | first unknown) and the offset of its block
-  // inverse; per unknown the row's off-node segment [begin, end); the
-  // segments' column indices in sweep (level-sorted) order
-  const longlong2 *tick;
-  const longlong2 *seg;
-  const int *cols;
   const int *fu;
   const int64_t *rowptr;
   const int *colidx;
@@ -676,62 +623,15 @@ struct TrsvArgs {
   int num_nodes;
   int Tr;              // local index of the energy row, -1 without energy
   int nvn;             // nodal fields per node
-  int *error;          // set when a wait gave up
-  long long spin_limit;  // polls before a wait gives up
 };
 
-// the "unpublished" sentinels: signalling NaNs (exponent all ones, quiet bit
-// clear, non-zero payload)
-static constexpr unsigned long long kUnpub64 = 0xFFF5DEAD5EEDF00DULL;
-static constexpr unsigned kUnpub32 = 0xFFA5EED5u;
-__device__ __forceinline__ bool unpublished(double v) {
-  return (unsigned long long)__double_as_longlong(v) == kUnpub64;
-}
-__device__ __forceinline__ bool unpublished(float v) { return __float_as_uint(v) == kUnpub32; }
-__device__ __forceinline__ void set_unpublished(double *p) {
-  *p = __longlong_as_double((long long)kUnpub64);
-}
-__device__ __forceinline__ void set_unpublished(float *p) { *p = __uint_as_float(kUnpub32); }
-
-__device__ __forceinline__ double ld_relaxed(const double *p) {
-  double v;
-  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_relaxed(const float *p) {
-  float v;
-  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(double *p, double v) {
-  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
-__device__ __forceinline__ void st_relaxed(float *p, float v) {
-  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
-}
-
-// fill a sweep's output with the sentinel
+// fills a sweep's output with the sentinel; resets the line sweeps' ticket
 template <class T>
-__global__ void trsv_prepare_kernel(int64_t n, T *x) {
+__global__ void trsv_prepare_kernel(int64_t n, T *x, int *ticket) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     set_unpublished(x + i);
-}
-
-// one solution value, polled until published (bounded; 0 once given up)
-template <class T>
-__device__ __forceinline__ T poll_value(const T *p, bool &gave_up, const int *error,
-                                        long long spin_limit) {
-  T v = ld_relaxed(p);
-  long long polls = 0;
-  while (unpublished(v)) {
-    if (gave_up || ++polls > spin_limit || ((polls & 1023) == 0 && *(volatile const int *)error)) {
-      gave_up = true;
-      return (T)0;
-    }
-    v = ld_relaxed(p);
-  }
-  return v;
 }
 
 // Dense inverses of every node's diagonal blocks of the factors: of the
@@ -780,7 +680,7 @@ __global__ void block_inverse_kernel(TrsvArgs g, const T *__restrict__ lu, T *__
   }
 }
 
-// Stage B, shared by the sweeps: lane r of the calling warp returns row r of
+// lane r of the calling warp returns row r of
 // D^-1 bv, D^-1 the node's block inverse (entry (r, c) at inv_s[c * 16 + r],
 // lower triangular for L, upper for U), bv the rows' right-hand sides less
 // their off-node parts; the products are added in column order.
@@ -794,232 +694,11 @@ __device__ __forceinline__ A node_block_apply(int lane, int nr, const A *inv_s, 
   return v;
 }
 
-// Copies every row's off-node segments of src into dst in the sweeps'
-// level-sorted order (entry p of a segment from segment start + rel[p]), so
-// the sync-free sweeps read factor values and column indices contiguously,
-// without the extra indirection.  One warp per row.
-template <class E>
-__global__ void sweep_gather_kernel(int N, const longlong2 *__restrict__ segL,
-                                    const longlong2 *__restrict__ segU,
-                                    const uint16_t *__restrict__ rel, const E *__restrict__ src,
-                                    E *__restrict__ dst) {
-  const int wpb = blockDim.x >> 5, lane = threadIdx.x & 31;
-  for (int i = blockIdx.x * wpb + (threadIdx.x >> 5); i < N; i += gridDim.x * wpb) {
-    for (int h = 0; h < 2; h++) {
-      const longlong2 sg = h ? segU[i] : segL[i];
-      for (int64_t p = sg.x + lane; p < sg.y; p += 32) dst[p] = src[sg.x + rel[p]];
-    }
-  }
-}
-
-template <class T, bool LOWER>
-__global__ void __launch_bounds__(kTrsvThreads, 4)
-    trsv_sync_free_kernel(TrsvArgs g, const T *__restrict__ lus, const T *__restrict__ binv,
-                          const T *__restrict__ b, T *x) {
-  using A = acc_t<T>;
-  constexpr int kPf = kPrefetchOf<T>;
-  __shared__ A bv[kMaxNodeDofs];                      // per row: rhs less the off-node part
-  __shared__ A inv_s[kMaxNodeDofs * kMaxNodeDofs];    // the node's block inverse, by column
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = kTrsvThreads / 32;
-  const unsigned nt = (unsigned)g.num_nodes, stride = gridDim.x;
-  unsigned t = blockIdx.x;
-  longlong2 tk = t < nt ? g.tick[t] : make_longlong2(0, 0);
-  for (; t < nt; t += stride) {
-    const int f0 = (int)(tk.x & 0xffffffffll), nr = (int)(tk.x >> 32);
-    const int64_t inv_off = tk.y;
-    // before polling: everything that does not depend on the sweep
-    A pv[kPf];
-    int pc[kPf];
-    int64_t pr0 = 0, pr1 = 0;
-    if (warp < nr) {
-      const longlong2 sg = g.seg[f0 + warp];
-      pr0 = sg.x;
-      pr1 = sg.y;
-#pragma unroll
-      for (int k = 0; k < kPf; k++) {
-        const int64_t p = pr0 + lane + 32 * k;
-        pv[k] = p < pr1 ? (A)lus[p] : (A)0;
-        pc[k] = p < pr1 ? g.cols[p] : -1;
-      }
-    }
-    for (int w = tid; w < nr * nr; w += kTrsvThreads) {
-      const int c = w / nr;
-      inv_s[c * kMaxNodeDofs + (w - c * nr)] = (A)binv[inv_off + w];
-    }
-    // this CTA's next node (static round-robin tickets)
-    if (t + stride < nt) tk = g.tick[t + stride];
-    // stage A
-    bool gave_up = false;
-    for (int r = warp; r < nr; r += NW) {
-      const A rhs_r = (A)__ldcg(b + f0 + r);
-      A s0 = 0;
-      int64_t p, p1;
-      if (r == warp) {
-        // the prefetched row: load all its values at once, then add them in
-        // the fixed (level-sorted, oldest first) order, each as soon as it
-        // and every earlier one are published -- the values published long
-        // ago are added while the newest ones are still awaited; a wait
-        // re-polls only the value it waits for, so waiting warps issue few
-        // instructions
-        A zv[kPf];
-        unsigned pending = 0;
-#pragma unroll
-        for (int k = 0; k < kPf; k++) {
-          zv[k] = 0;
-          if (pc[k] >= 0) {
-            const T v = ld_relaxed(x + pc[k]);
-            if (unpublished(v)) pending |= 1u << k; else zv[k] = (A)v;
-          }
-        }
-        long long polls = 0;
-#pragma unroll
-        for (int k = 0; k < kPf; k++) {
-          while (!gave_up && (pending & (1u << k))) {
-            if (++polls > g.spin_limit ||
-                ((polls & 1023) == 0 && *(volatile const int *)g.error)) {
-              gave_up = true;
-              break;
-            }
-            const T v = ld_relaxed(x + pc[k]);
-            if (!unpublished(v)) {
-              zv[k] = (A)v;
-              pending &= ~(1u << k);
-            }
-          }
-          if (pc[k] >= 0) s0 = fmx(pv[k], zv[k], s0);
-        }
-        p = pr0 + lane + 32 * kPf;
-        p1 = pr1;
-      } else {
-        const longlong2 sg = g.seg[f0 + r];
-        p = sg.x + lane;
-        p1 = sg.y;
-      }
-      for (; p < p1; p += 32)
-        s0 = fmx((A)lus[p], (A)poll_value(x + g.cols[p], gave_up, g.error, g.spin_limit), s0);
-      const A sum = wsum(s0);
-      if (lane == 0) bv[r] = rhs_r - sum;
-    }
-    if (__syncthreads_or(gave_up) && tid == 0) atomicExch(g.error, 1);
-    // stage B
-    if (warp == 0) {
-      const A v = node_block_apply<A, LOWER>(lane, nr, inv_s, bv);
-      if (lane < nr) st_relaxed(x + f0 + lane, (T)v);
-    }
-    __syncthreads();
-  }
-}
-
-// The same sweep with one warp per node, for meshes whose nodes have few
-// unknowns and short rows (QUAD9 problems: 2-6 rows of at most a few dozen
-// off-node entries).  A node's rows go to lane groups of G = 32 / R lanes
-// (R: the row count rounded up to a power of two), a group sums its row in
-// a fixed order (lane by lane, then a butterfly within the group), and the
-// block inverse is applied with one shuffle per row -- no shared memory and
-// no barrier, so a warp needs far fewer resources than a CTA and many more
-// nodes are in flight (each 128-thread CTA holds four).  Warp w of the grid
-// takes tickets w, w + W, ... (W warps in all), with the same progress
-// argument as the CTA sweep.  Used when every node has at most kWarpMaxRows
-// rows and every row's off-node segment fits its group's prefetch window:
-// always in FP32, in FP64 only for wide levels (Solver::init).
-static constexpr int kWarpMaxRows = 8;
-static constexpr int kPrefetchW = 8;
-static constexpr int kWarpSweepThreads = 128;
-
-template <class T, bool LOWER>
-__global__ void __launch_bounds__(kWarpSweepThreads)
-    trsv_sync_free_warp_kernel(TrsvArgs g, const T *__restrict__ lus,
-                               const T *__restrict__ binv, const T *__restrict__ b, T *x) {
-  using A = acc_t<T>;
-  const int lane = threadIdx.x & 31;
-  const unsigned nt = (unsigned)g.num_nodes;
-  const unsigned wpb = blockDim.x >> 5, stride = gridDim.x * wpb;
-  unsigned t = blockIdx.x * wpb + (threadIdx.x >> 5);
-  longlong2 tk = t < nt ? g.tick[t] : make_longlong2(0, 0);
-  for (; t < nt; t += stride) {
-    const int f0 = (int)(tk.x & 0xffffffffll), nr = (int)(tk.x >> 32);
-    const int64_t inv_off = tk.y;
-    int R = 1;
-    while (R < nr) R <<= 1;
-    const int G = 32 / R;                     // lanes per row
-    const int r = lane / G, gl = lane - r * G;
-    const bool act = r < nr;
-    A pv[kPrefetchW];
-    int pc[kPrefetchW];
-    int64_t pr0 = 0, pr1 = 0;
-    if (act) {
-      const longlong2 sg = g.seg[f0 + r];
-      pr0 = sg.x;
-      pr1 = sg.y;
-    }
-#pragma unroll
-    for (int k = 0; k < kPrefetchW; k++) {
-      const int64_t p = pr0 + gl + (int64_t)G * k;
-      pv[k] = p < pr1 ? (A)lus[p] : (A)0;
-      pc[k] = p < pr1 ? g.cols[p] : -1;
-    }
-    // lane c < nr holds row c of the block inverse
-    A dv[kWarpMaxRows];
-#pragma unroll
-    for (int c = 0; c < kWarpMaxRows; c++)
-      dv[c] = (lane < nr && c < nr) ? (A)binv[inv_off + (int64_t)c * nr + lane] : (A)0;
-    const A rhs_r = act ? (A)__ldcg(b + f0 + r) : (A)0;
-    if (t + stride < nt) tk = g.tick[t + stride];
-    // stage A: the row's off-node sum, values added in the fixed order as
-    // they arrive (a wait re-polls only its own value)
-    bool gave_up = false;
-    A zv[kPrefetchW];
-    unsigned pending = 0;
-#pragma unroll
-    for (int k = 0; k < kPrefetchW; k++) {
-      zv[k] = 0;
-      if (pc[k] >= 0) {
-        const T v = ld_relaxed(x + pc[k]);
-        if (unpublished(v)) pending |= 1u << k; else zv[k] = (A)v;
-      }
-    }
-    A s0 = 0;
-    long long polls = 0;
-#pragma unroll
-    for (int k = 0; k < kPrefetchW; k++) {
-      while (!gave_up && (pending & (1u << k))) {
-        if (++polls > g.spin_limit || ((polls & 1023) == 0 && *(volatile const int *)g.error)) {
-          gave_up = true;
-          break;
-        }
-        const T v = ld_relaxed(x + pc[k]);
-        if (!unpublished(v)) {
-          zv[k] = (A)v;
-          pending &= ~(1u << k);
-        }
-      }
-      if (pc[k] >= 0) s0 = fmx(pv[k], zv[k], s0);
-    }
-    for (int64_t p = pr0 + gl + (int64_t)G * kPrefetchW; p < pr1; p += G)
-      s0 = fmx((A)lus[p], (A)poll_value(x + g.cols[p], gave_up, g.error, g.spin_limit), s0);
-    for (int o = G >> 1; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    const A bvr = rhs_r - s0;
-    // stage B: x_n = D^-1 (rhs - off-node part), products in column order
-    A v = 0;
-#pragma unroll
-    for (int c = 0; c < kWarpMaxRows; c++) {
-      if (c < nr) {
-        const A bc = __shfl_sync(0xffffffffu, bvr, c * G);
-        if (lane < nr && (LOWER ? c <= lane : c >= lane)) v = fmx(dv[c], bc, v);
-      }
-    }
-    if (lane < nr) st_relaxed(x + f0 + lane, (T)v);
-    if (__any_sync(0xffffffffu, gave_up) && lane == 0) atomicExch(g.error, 1);
-  }
-}
-
 // One dependency level of a triangular sweep, one CTA per node: the nodes of
 // a level do not depend on each other, so the launch boundary is the only
-// synchronisation.  Same two stages as the sync-free sweep (rows over the
-// warps, then the in-node solve over the lanes of warp 0), in place on z;
-// used for short level schedules (the multicoloured order), launched level
-// after level from a captured graph.
+// synchronisation.  The rows go over the warps, then the block inverse over
+// the lanes of warp 0, in place on z; used for short level schedules (the
+// multicoloured order), launched level after level from a captured graph.
 template <class T, bool LOWER>
 __global__ void __launch_bounds__(kTrsvThreads)
     trsv_level_cta_kernel(const int *__restrict__ nodes, TrsvArgs g, const T *__restrict__ lu,
@@ -1064,13 +743,9 @@ __global__ void __launch_bounds__(kTrsvThreads)
   }
 }
 
-// the sweeps' view of the preconditioner layout (the sync-free sweep sets
-// its tickets, segments and columns)
+// the sweeps' view of the preconditioner layout
 static TrsvArgs trsv_args(const Solver *S) {
   TrsvArgs g;
-  g.tick = nullptr;
-  g.seg = nullptr;
-  g.cols = nullptr;
   g.fu = S->P.fu;
   g.rowptr = S->P.rowptr;
   g.colidx = S->P.colidx;
@@ -1079,8 +754,6 @@ static TrsvArgs trsv_args(const Solver *S) {
   g.num_nodes = S->C->L.num_nodes;
   g.Tr = S->C->L.energy ? S->C->L.dim : -1;
   g.nvn = S->C->L.nvn;
-  g.error = nullptr;
-  g.spin_limit = S->C->sweep_spin_limit > 0 ? S->C->sweep_spin_limit : kSpinLimit;
   return g;
 }
 
@@ -1135,12 +808,17 @@ void build_ilu_schedule(const Layout &L, IluSchedule &S) {
 Solver::~Solver() {
   if (prec64) cudaGraphExecDestroy(prec64);
   if (prec32) cudaGraphExecDestroy(prec32);
-  void *p[] = {d_lu, d_lu32, d_lus, d_lus32, d_binv, d_binv32, d_Z, d_a32, d_diag, d_lo_nodes, d_up_nodes, d_scale, d_work, d_flags,
+  void *p[] = {d_lu, d_lu32, d_binv, d_binv32, d_Z, d_a32, d_diag, d_lo_nodes, d_up_nodes, d_scale, d_work, d_flags,
                d_sweep_y, d_V, d_V32, d_t, d_w, d_r, d_xs, d_t32, d_w32};
   for (void *q : p)
     if (q) cudaFree(q);
   for (void *q : owned)
     if (q) cudaFree(q);
+  void *lp[] = {d_line_lo, d_line_up, d_line_lo32, d_line_up32};
+  for (void *q : lp)
+    if (q) cudaFree(q);
+  line_lo.release();
+  line_up.release();
   if (h_work) cudaFreeHost(h_work);
   if (h_segout) cudaFreeHost(h_segout);
 }
@@ -1247,80 +925,10 @@ int Solver::init(Context *c, int krylov) {
   up_ptr = S.up_ptr;
   num_levels = (int)lo_ptr.size() - 1;
   {
-    std::vector<uint16_t> rel;
-    if (build_sweep_order(*LP, S.lev, S.levu, rel)) return fail("a matrix row is too long for the sweeps");
-    GB_CU(cudaMalloc(&d_sweep_rel, sizeof(uint16_t) * rel.size()), "sweep order");
-    owned.push_back(d_sweep_rel);
-    GB_CU(cudaMemcpy(d_sweep_rel, rel.data(), sizeof(uint16_t) * rel.size(),
-                     cudaMemcpyHostToDevice), "sweep order");
-  }
-  {
-    // the sync-free sweeps' tables: every row's off-node segments, the
-    // tickets of both sweeps, and the column indices in sweep order
-    const int Tr = L.energy ? L.dim : -1;
-    std::vector<longlong2> sl(N), su(N);
-    for (int n = 0; n < LP->num_nodes; n++) {
-      const int f0 = LP->fu[n], nr = LP->fu[n + 1] - f0;
-      for (int r = 0; r < nr; r++) {
-        const int i = f0 + r;
-        auto b = LP->colidx.begin() + LP->rowptr[i], e = LP->colidx.begin() + LP->rowptr[i + 1];
-        const int64_t di = (int64_t)(std::lower_bound(b, e, i) - LP->colidx.begin());
-        const int na = (r == Tr ? L.nvn : nr) - 1 - r;
-        sl[i] = make_longlong2(LP->rowptr[i], di - r);
-        su[i] = make_longlong2(di + 1 + na, LP->rowptr[i + 1]);
-      }
-    }
-    // one warp per node when every node has at most kWarpMaxRows rows and
-    // every row's off-node segments fit its lane group's prefetch window
-    {
-      bool fits = true;
-      for (int n = 0; n < LP->num_nodes && fits; n++) {
-        const int f0 = LP->fu[n], nr = LP->fu[n + 1] - f0;
-        int R = 1;
-        while (R < nr) R <<= 1;
-        const int64_t cap = (int64_t)(32 / R) * kPrefetchW;
-        if (nr > kWarpMaxRows) fits = false;
-        for (int r = 0; r < nr && fits; r++)
-          if (sl[f0 + r].y - sl[f0 + r].x > cap || su[f0 + r].y - su[f0 + r].x > cap) fits = false;
-      }
-      // FP32 sweeps take the warp form whenever it fits; FP64 ones only when
-      // the levels are wide (several independent problems interleaved), as
-      // the FP64 warp form's 85 registers a thread cost more than its
-      // shorter critical path saves on a single mesh
-      warp_sweep32 = fits;
-      warp_sweep64 = fits && LP->num_nodes > 300LL * (int64_t)lo_ptr.size();
-    }
-    auto ticks = [&](const std::vector<int> &order, bool upper) {
-      std::vector<longlong2> tk(order.size());
-      for (size_t t = 0; t < order.size(); t++) {
-        const int n = order[t], f0 = LP->fu[n];
-        const long long nr = LP->fu[n + 1] - f0;
-        tk[t] = make_longlong2((nr << 32) | (long long)f0, ip[n] + (upper ? nr * nr : 0));
-      }
-      return tk;
-    };
-    auto upv = [&](const auto &vec, auto **dst, const char *what) -> int {
-      GB_CU(cudaMalloc((void **)dst, sizeof(vec[0]) * vec.size()), what);
-      owned.push_back(*dst);
-      GB_CU(cudaMemcpy(*dst, vec.data(), sizeof(vec[0]) * vec.size(), cudaMemcpyHostToDevice),
-            what);
-      return 0;
-    };
-    if (upv(sl, &d_segL, "sweep segments") || upv(su, &d_segU, "sweep segments") ||
-        upv(ticks(S.lo_nodes, false), &d_tick_lo, "sweep tickets") ||
-        upv(ticks(S.up_nodes, true), &d_tick_up, "sweep tickets"))
-      return -1;
-    {
-      std::vector<int> rev(S.lo_nodes.rbegin(), S.lo_nodes.rend());
-      if (upv(ticks(rev, false), &d_tick_lo_rev, "sweep tickets")) return -1;
-    }
-    GB_CU(cudaMalloc(&d_sweep_cols, sizeof(int) * (size_t)nnz), "sweep columns");
-    owned.push_back(d_sweep_cols);
-    GB_CU(cudaMemset(d_sweep_cols, 0, sizeof(int) * (size_t)nnz), "sweep columns");
-    sweep_gather_kernel<int><<<(N + 7) / 8, 256>>>(N, d_segL, d_segU, d_sweep_rel, P.colidx,
-                                                   d_sweep_cols);
-    GB_CU(cudaGetLastError(), "sweep columns");
-    GB_CU(cudaDeviceSynchronize(), "sweep columns");
+    LineTables lo, hi;
+    if (build_line_tables(*LP, false, lo) || build_line_tables(*LP, true, hi))
+      return fail("a matrix row is too long for the sweeps");
+    if (line_lo.upload(lo) || line_up.upload(hi)) return -1;
   }
   GB_CU(cudaMalloc(&d_lo_nodes, sizeof(int) * S.lo_nodes.size()), "sched");
   GB_CU(cudaMemcpy(d_lo_nodes, S.lo_nodes.data(), sizeof(int) * S.lo_nodes.size(),
@@ -1449,6 +1057,21 @@ static cudaError_t capture_prec(Solver *S, const T *lu, const T *binv, T *z, cud
   return e;
 }
 
+// the block inverses and the line sweeps' scaled factors
+template <class T>
+static int gather_lines(Solver *S, const TrsvArgs &a, const T *lu, T *binv, T **lo, T **up,
+                        cudaStream_t st) {
+  if (!*lo)
+    GB_CU(cudaMalloc(lo, sizeof(T) * 32 * (size_t)S->line_lo.num_groups), "sweep factors");
+  if (!*up)
+    GB_CU(cudaMalloc(up, sizeof(T) * 32 * (size_t)S->line_up.num_groups), "sweep factors");
+  block_inverse_kernel<T><<<(S->C->L.num_nodes + 7) / 8, 256, 0, st>>>(a, lu, binv);
+  const LineFactors F{S->P.fu, S->P.rowptr, S->d_inv_ptr, a.Tr};
+  GB_CU(line_gather<T>(S->line_lo, false, F, lu, binv, *lo, st), "sweep factors");
+  GB_CU(line_gather<T>(S->line_up, true, F, lu, binv, *up, st), "sweep factors");
+  return 0;
+}
+
 int Solver::factor(const double *vals, bool fp32, cudaStream_t st) {
   d_A = vals;
   int *nfix = (int *)(d_work + kRedBlocks * 3 + 10);
@@ -1500,32 +1123,18 @@ int Solver::factor(const double *vals, bool fp32, cudaStream_t st) {
   GB_CU(cudaGetLastError(), "ILU(0) factorisation");
   {
     const TrsvArgs a = trsv_args(this);
-    const int gs = (N + 7) / 8;
-    if (fp32) {
-      if (!d_binv32) GB_CU(cudaMalloc(&d_binv32, sizeof(float) * inv_len), "block inverses");
-      if (!d_lus32) GB_CU(cudaMalloc(&d_lus32, sizeof(float) * nnz), "sweep-ordered factors");
-      block_inverse_kernel<float><<<(C->L.num_nodes + 7) / 8, 256, 0, st>>>(a, d_lu32, d_binv32);
-      sweep_gather_kernel<float><<<gs, 256, 0, st>>>(N, d_segL, d_segU, d_sweep_rel, d_lu32,
-                                                     d_lus32);
-    } else {
-      if (!d_lus) GB_CU(cudaMalloc(&d_lus, sizeof(double) * nnz), "sweep-ordered factors");
-      block_inverse_kernel<double><<<(C->L.num_nodes + 7) / 8, 256, 0, st>>>(a, d_lu, d_binv);
-      sweep_gather_kernel<double><<<gs, 256, 0, st>>>(N, d_segL, d_segU, d_sweep_rel, d_lu,
-                                                      d_lus);
-    }
+    if (fp32 && !d_binv32)
+      GB_CU(cudaMalloc(&d_binv32, sizeof(float) * inv_len), "block inverses");
+    if (fp32 ? gather_lines<float>(this, a, d_lu32, d_binv32, &d_line_lo32, &d_line_up32, st)
+             : gather_lines<double>(this, a, d_lu, d_binv, &d_line_lo, &d_line_up, st))
+      return -1;
     GB_CU(cudaGetLastError(), "block inverses");
   }
   if (fp32) {
     to_f32_kernel<<<1216, 256, 0, st>>>(nnz, vals, d_a32);
     GB_CU(cudaGetLastError(), "FP32 matrix copy");
-    if (!prec32 && use_level_graph())
-      GB_CU(capture_prec<float>(this, d_lu32, d_binv32, ordering ? d_tp32 : d_t32, st, &prec32),
-            "ILU32 graph");
     have_lu32 = true;
   } else {
-    if (!prec64 && use_level_graph())
-      GB_CU(capture_prec<double>(this, d_lu, d_binv, ordering ? d_tp : d_t, st, &prec64),
-            "ILU graph");
     have_lu64 = true;
   }
   return 0;
@@ -1557,73 +1166,45 @@ int Solver::copy_factors(double *host, bool fp32, cudaStream_t st) {
 }
 
 template <class T>
-static int sync_free_apply(Solver *S, const T *lus, const T *binv, T *z, cudaStream_t st) {
+static int sync_free_apply(Solver *S, T *z, cudaStream_t st) {
   if (!S->d_flags) {
     GB_CU(cudaMalloc(&S->d_flags, 16 * sizeof(unsigned)), "trsv error word");
     GB_CU(cudaMemsetAsync(S->d_flags, 0, 16 * sizeof(unsigned), st), "trsv error word");
     GB_CU(cudaMalloc(&S->d_sweep_y, sizeof(double) * (size_t)S->N), "trsv scratch");
-    int per_sm = 1 << 30, dev = 0, sms = 0;
-    const void *fns[4] = {(const void *)trsv_sync_free_kernel<double, true>,
-                          (const void *)trsv_sync_free_kernel<double, false>,
-                          (const void *)trsv_sync_free_kernel<float, true>,
-                          (const void *)trsv_sync_free_kernel<float, false>};
-    const void *wfns[4] = {(const void *)trsv_sync_free_warp_kernel<double, true>,
-                           (const void *)trsv_sync_free_warp_kernel<double, false>,
-                           (const void *)trsv_sync_free_warp_kernel<float, true>,
-                           (const void *)trsv_sync_free_warp_kernel<float, false>};
-    int wper_sm = 1 << 30;
-    for (const void *f : fns) {
-      int b = 0;
-      GB_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kTrsvThreads, 0), "occupancy");
-      per_sm = std::min(per_sm, b);
-    }
-    for (const void *f : wfns) {
-      int b = 0;
-      GB_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kWarpSweepThreads, 0),
-            "occupancy");
-      wper_sm = std::min(wper_sm, b);
-    }
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    S->trsv_grid = std::max(1, per_sm) * sms;
-    S->trsv_grid_warp = std::max(1, wper_sm) * sms;
-    S->prep_grid = 2 * sms;
+    cudaDeviceGetAttribute(&S->num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  TrsvArgs g = trsv_args(S);  // the tickets and segments are set per sweep below
-  g.error = (int *)(S->d_flags + 4);
-  g.cols = S->d_sweep_cols;
   T *y = static_cast<T *>(S->d_sweep_y);
-  // the host-injected fault of gb_set_sweep_fault: the lower sweep's nodes in
+  LineArgs a{};
+  a.error = (int *)(S->d_flags + 4);
+  a.ticket = (int *)(S->d_flags + 8);
+  a.spin_limit = S->C->sweep_spin_limit > 0 ? S->C->sweep_spin_limit : kSpinLimit;
+  const T *vl = sizeof(T) == 4 ? (const T *)S->d_line_lo32 : (const T *)S->d_line_lo;
+  const T *vu = sizeof(T) == 4 ? (const T *)S->d_line_up32 : (const T *)S->d_line_up;
+  // the host-injected fault of gb_set_sweep_fault: the lower sweep's lines in
   // reverse order (every dependency after its dependant) on one CTA, whose
   // first wait can then only end by running out
-  const longlong2 *lo_tick = S->d_tick_lo;
-  const bool warp = sizeof(T) == 4 ? S->warp_sweep32 : S->warp_sweep64;
-  int grid = warp ? S->trsv_grid_warp : S->trsv_grid;
-  if (S->C->sweep_reverse_lower) {
-    lo_tick = S->d_tick_lo_rev;
-    grid = 1;
-  }
+  const bool rev = S->C->sweep_reverse_lower != 0;
   // L: z -> y, then U: y -> z; each output starts all unpublished
-  trsv_prepare_kernel<T><<<S->prep_grid, 256, 0, st>>>(S->N, y);
-  g.tick = lo_tick;
-  g.seg = S->d_segL;
-  if (warp)
-    trsv_sync_free_warp_kernel<T, true><<<grid, kWarpSweepThreads, 0, st>>>(g, lus, binv, z, y);
-  else
-    trsv_sync_free_kernel<T, true><<<grid, kTrsvThreads, 0, st>>>(g, lus, binv, z, y);
-  trsv_prepare_kernel<T><<<S->prep_grid, 256, 0, st>>>(S->N, z);
-  g.tick = S->d_tick_up;
-  g.seg = S->d_segU;
-  if (warp)
-    trsv_sync_free_warp_kernel<T, false><<<grid, kWarpSweepThreads, 0, st>>>(g, lus, binv, y, z);
-  else
-    trsv_sync_free_kernel<T, false><<<grid, kTrsvThreads, 0, st>>>(g, lus, binv, y, z);
+  const int prep = 2 * S->num_sms;
+  a.lines = rev ? S->line_lo.d_lines_rev : S->line_lo.d_lines;
+  trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, y, a.ticket);
+  GB_CU(line_sweep<T>(S->line_lo, a, vl, z, y, S->num_sms, rev, st), "trsv");
+  a.lines = S->line_up.d_lines;
+  trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, z, a.ticket);
+  GB_CU(line_sweep<T>(S->line_up, a, vu, y, z, S->num_sms, false, st), "trsv");
   GB_CU(cudaGetLastError(), "trsv");
   return 0;
 }
 
+// The line sweeps are the faster ones on every schedule measured, short ones
+// included (us per GMRES iteration, lines / graph, FP64): 4 x 4 cavity 166 /
+// 289, 2^3 cube 193 / 456, and in the multicoloured order 32 x 32 cavity 184 /
+// 193, 8^3 cube 240 / 519, 16^3 cube 506 / 950.  The graph serves when it is
+// asked for.
 bool Solver::use_level_graph() const {
-  return C->trsv == 1 || (C->trsv == 2 && num_levels <= kMaxGraphLevels);
+  return C->trsv == 1;
 }
 
 int Solver::check_trsv_error() {
@@ -1638,15 +1219,14 @@ int Solver::check_trsv_error() {
 }
 
 template <class T>
-static int apply_prec(Solver *S, const T *lus, const T *binv, T *t, T *tp,
-                      cudaGraphExec_t graph, cudaStream_t st) {
+static int apply_prec(Solver *S, T *t, T *tp, cudaGraphExec_t graph, cudaStream_t st) {
   T *z = t;
   if (S->ordering == 1) {  // t -> P t, solve, P^T
     gather_kernel<T><<<304, 256, 0, st>>>(S->N, S->d_umap, t, tp);
     z = tp;
   }
   if (!S->use_level_graph()) {
-    if (sync_free_apply<T>(S, lus, binv, z, st)) return -1;
+    if (sync_free_apply<T>(S, z, st)) return -1;
   } else {
     GB_CU(cudaGraphLaunch(graph, st), "ILU apply");
   }
@@ -1656,10 +1236,16 @@ static int apply_prec(Solver *S, const T *lus, const T *binv, T *t, T *tp,
 }
 
 int Solver::apply_prec64(cudaStream_t st) {
-  return apply_prec<double>(this, d_lus, d_binv, d_t, d_tp, prec64, st);
+  if (use_level_graph() && !prec64)
+    GB_CU(capture_prec<double>(this, d_lu, d_binv, ordering ? d_tp : d_t, st, &prec64),
+          "ILU graph");
+  return apply_prec<double>(this, d_t, d_tp, prec64, st);
 }
 int Solver::apply_prec32(cudaStream_t st) {
-  return apply_prec<float>(this, d_lus32, d_binv32, d_t32, d_tp32, prec32, st);
+  if (use_level_graph() && !prec32)
+    GB_CU(capture_prec<float>(this, d_lu32, d_binv32, ordering ? d_tp32 : d_t32, st, &prec32),
+          "ILU32 graph");
+  return apply_prec<float>(this, d_t32, d_tp32, prec32, st);
 }
 
 // ------------------------------------------------------------ helpers

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "gb_layout.h"
+#include "gb_sweep.h"
 
 namespace gb {
 
@@ -71,18 +72,14 @@ struct Solver {
   float *d_binv32 = nullptr;
   int64_t *d_inv_ptr = nullptr;
   int64_t inv_len = 0;
-  // the sync-free sweeps' tables (see trsv_sync_free_kernel): factors and
-  // column indices in sweep order, per-row off-node segments, tickets
-  double *d_lus = nullptr;
-  float *d_lus32 = nullptr;
-  int *d_sweep_cols = nullptr;
-  longlong2 *d_segL = nullptr, *d_segU = nullptr;
-  longlong2 *d_tick_lo = nullptr, *d_tick_up = nullptr, *d_tick_lo_rev = nullptr;
+  // the sync-free sweeps' tables and scaled factors (gb_sweep.cu)
+  LineSweep line_lo, line_up;
+  double *d_line_lo = nullptr, *d_line_up = nullptr;
+  float *d_line_lo32 = nullptr, *d_line_up32 = nullptr;
   int64_t *d_diag = nullptr;    // position of the diagonal in every row
   int *d_fu = nullptr;          // first unknown per node (shared with C)
   int *d_lo_nodes = nullptr, *d_up_nodes = nullptr;
   std::vector<int> lo_ptr, up_ptr;
-  uint16_t *d_sweep_rel = nullptr; // level-sorted entry order of the sweeps (build_sweep_order)
   const double *d_A = nullptr;  // scaled FP64 matrix the factors were built from
   double pivot_tau = 1e-4;      // ILU(0) pivot floor on the row-scaled matrix
   int maxnb = 0, lmax = 0;      // largest node neighbourhood / block-row length
@@ -98,14 +95,10 @@ struct Solver {
   cudaGraphExec_t prec64 = nullptr, prec32 = nullptr;  // captured ILU solves on d_t / d_t32
   unsigned *d_flags = nullptr;  // sync-free sweeps: [4] error word
   void *d_sweep_y = nullptr;    // sync-free sweeps: the L sweep's output (N values)
-  int trsv_grid = 0, prep_grid = 0;
-  int trsv_grid_warp = 0;
-  // sync-free sweeps with one warp per node (short rows), per precision
-  bool warp_sweep32 = false, warp_sweep64 = false;
+  int num_sms = 0;
   int check_trsv_error();
   // level-scheduled sweeps from a captured graph (else the sync-free ones)
   bool use_level_graph() const;
-  static constexpr int kMaxGraphLevels = 64;  // automatic mode: graph up to this depth
   ~Solver();
   int init(Context *c, int krylov);
   // ILU(0) factors of the scaled matrix vals (FP64, or FP32 with the FP32

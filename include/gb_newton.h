@@ -57,14 +57,13 @@ int gb_msr_pattern_host(const gb_problem_desc *desc, int *ija, long long *msr_le
  * (nnz).  Any output may be NULL. */
 int gb_ilu_permutation_host(const gb_problem_desc *desc, int *perm, int *num_colours, int *umap,
                             long long *rowptr, int *colidx, long long *vmap);
-/* Host only: the order in which the sync-free ILU(0) sweeps add each row's
- * off-node entries (oldest dependency level first) for the given node
- * ordering (GB_ILU_*), in the CSR layout of that ordering (the permuted one
- * of gb_ilu_permutation_host for GB_ILU_MULTICOLOUR): entry p of a row's
- * off-node lower or upper segment is read from the segment's start +
- * rel[p] (nnz values); lev / levu (num_nodes, may be NULL) get every
- * node's forward / backward dependency level.  For inspecting the sweeps;
- * no counterpart in the reference. */
+/* Host only: every row's off-node entries by dependency level (oldest
+ * first) for the given node ordering (GB_ILU_*), in the CSR layout of that
+ * ordering (the permuted one of gb_ilu_permutation_host for
+ * GB_ILU_MULTICOLOUR): entry p of a row's off-node lower or upper segment is
+ * at the segment's start + rel[p] (nnz values); lev / levu (num_nodes, may
+ * be NULL) get every node's forward / backward dependency level.  For
+ * inspecting the schedule; no counterpart in the reference. */
 int gb_sweep_order_host(const gb_problem_desc *desc, int ordering, unsigned short *rel,
                         int *lev, int *levu);
 /* CSR pattern used on the device: rowptr (N+1, int64), colidx (nnz). */
@@ -163,12 +162,11 @@ int gb_set_ilu_ordering(gb_ctx *ctx, int ordering);
 int gb_set_element_density(gb_ctx *ctx, const double *rho);
 
 /* ILU(0) triangular solves of later linear solves: 0 = sync-free sweeps
- * (one launch per factor; each node polls the solution values it depends
- * on, bounded, then publishes its own; a CTA per node, or a warp per node
- * on meshes with short rows), 1 = level-scheduled sweeps (one launch per
- * dependency level, a CTA per node) replayed as a CUDA graph, 2 = automatic
- * (the default: the graph when the schedule has at most 64 levels, as in
- * the multicoloured order; the sync-free sweeps otherwise).  All give the
+ * (one launch per factor; a CTA takes a line of consecutive nodes and polls
+ * the solution values of other lines, bounded, while it publishes its own),
+ * 1 = level-scheduled sweeps (one launch per dependency level, a CTA per
+ * node) replayed as a CUDA graph, 2 = automatic (the default: the sync-free
+ * sweeps, which are the faster ones in both node orders).  All give the
  * same result to rounding.  No counterpart in the reference (AztecOO's ILU
  * solves are sequential). */
 int gb_set_triangular_solve(gb_ctx *ctx, int mode);
@@ -176,14 +174,13 @@ int gb_set_triangular_solve(gb_ctx *ctx, int mode);
 /* Host-side fault injection for the sync-free sweeps' bounded waits; no
  * counterpart in the reference.  spin_limit sets the polls a wait makes
  * before it gives up (<= 0: the default, 2^22, about 0.3 s).  With
- * reverse_lower != 0 the lower sweep hands its nodes out in reverse order
- * (every dependency after the node that needs it) on a grid of one CTA,
+ * reverse_lower != 0 the lower sweep hands its lines out in reverse order
+ * (every dependency after the line that needs it) on a grid of one CTA,
  * so its first wait can only end by running out: the sweep then finishes
  * with the error word set, later waits of the solve stop within 1024 polls,
  * and the linear solve returns -1 ("a dependency wait gave up") with the
  * context still usable.  (0, 0) restores the normal sweeps.  Applies to
- * the sync-free sweeps only (gb_set_triangular_solve mode 0, or 2 with a
- * deep schedule). */
+ * the sync-free sweeps only (gb_set_triangular_solve modes 0 and 2). */
 int gb_set_sweep_fault(gb_ctx *ctx, long long spin_limit, int reverse_lower);
 
 /* Replaces the material of a context (same mesh, DOF map and pattern), as
