@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gb_context.h"
+#include "gb_factor.h"
 #include "gb_publish.cuh"
 #include "gb_solve.h"
 
@@ -300,300 +301,6 @@ __global__ void spmv_kernel(int N, const int64_t *__restrict__ rowptr,
 
 // ------------------------------------------------------------ ILU(0)
 
-// first position in [lo, hi) of a sorted column list holding c, or -1
-__device__ __forceinline__ int64_t find_col(const int *__restrict__ colidx, int64_t lo, int64_t hi,
-                                            int c) {
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (colidx[mid] < c)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
-}
-
-// ILU(0) of the rows of one node per CTA, all nodes of one level at once.
-//
-// The pattern is dense in node blocks (every unknown of a node couples with
-// every unknown of every neighbour node; the energy row alone skips pressure
-// columns), so the reference's scalar ILU(0) in node-major order is, block
-// by block: for each lower neighbour node m (ascending)
-//     L_nm   = A_nm U_mm^-1                 (triangular, <= 16 x 16)
-//     A_nq  -= L_nm U_mq   for every q > m neighbouring both n and m
-// then the dense elimination of the node's own diagonal block and the rest
-// of its row.  Fill outside the pattern (energy row x pressure column) is
-// dropped, as in ILU(0).  The node's block row lives in shared memory; the
-// factored rows of lower nodes are read from global memory (earlier levels).
-// A pivot smaller than tau in magnitude (the row-scaled matrix has unit row
-// sums) becomes +-tau: in the reference's node-major order an element
-// without a pressure datum whose earlier velocity unknowns are all Dirichlet
-// rows leaves an exactly singular pressure pivot.
-// unknowns per node: nodal fields (<= 3 + 1 + GB_MAX_SPECIES) + P1 pressures
-static constexpr int kMaxNodeDofs = 16;
-
-struct IluArgs {
-  const int *fu;
-  const int64_t *rowptr;
-  const int *nbr_ptr, *nbr_node, *nbr_off, *nbr_offT;
-  const int *nbr_self;  // every node's own position in its neighbour list
-  int dim, nvn, energy;
-  int maxnb, lmax, maxnr;
-  double tau;
-  int *nfix;
-};
-
-// Shared memory of one ilu0_block_kernel CTA (element type of size tsize).
-static size_t ilu_smem_bytes(size_t tsize, int maxnb, int maxnr, int lmax) {
-  return sizeof(int64_t) * (size_t)maxnb * maxnr +                          // srow
-         tsize * ((size_t)maxnr * lmax + 3 * kMaxNodeDofs * kMaxNodeDofs + 2 * kMaxNodeDofs) +
-         sizeof(int) * (15 * (size_t)maxnb + 4);
-}
-
-// ILU(0) of one node's block row (one CTA per node, the nodes of one
-// dependency level per launch).  The block row of node n -- its rows over
-// the columns of all its neighbours -- lives in shared memory.  For every
-// lower neighbour m, in increasing order:
-//   step 1  L_nm = A_nm U_mm^-1   (U_mm: m's diagonal block, already final)
-//   step 2  A_nq -= L_nm U_mq     for every neighbour q > m of m that is
-//                                 also a neighbour of n
-// then the diagonal block is factorised in place and the row written back.
-// Everything that depends only on the node graph and on finished nodes is
-// loaded up front for all m at once (their neighbour-list bounds, own
-// positions and row starts).  Per m, "round A" loads m's neighbour list
-// (each neighbour's slot in n's list found by binary search in shared
-// memory, the shared ones listed through a shared-memory counter), U_mm and
-// its reciprocal pivots; it only reads finished nodes, so round A of m+1
-// runs during step 2 of m, into the other half of double-buffered tables.
-// Step 2 gives each thread one (shared neighbour, column) pair: it loads
-// that column of U_mq once and updates every row of n (each target is
-// updated once per m, so the list order does not matter).
-struct IluRoundA {
-  int *tslot, *toff, *toffT, *plist, *np;
-};
-
-template <class T>
-__device__ __forceinline__ void ilu_round_a(const IluArgs &g, int tid, int nt, int m, int mb,
-                                            int mnb, int nm, int Tr, const int64_t *mrow,
-                                            int moff, int moffT, const int *snb, int nb,
-                                            const T *__restrict__ lu, IluRoundA bufs, T *umm,
-                                            T *rdm) {
-  for (int t = tid; t < mnb; t += nt) {
-    const int q = g.nbr_node[mb + t];
-    int slot = -1;
-    if (q > m) {
-      int lo = 0, hi = nb - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (snb[mid] < q) lo = mid + 1; else hi = mid;
-      }
-      if (snb[lo] == q) slot = lo;
-    }
-    bufs.tslot[t] = slot;
-    if (slot >= 0) {
-      bufs.toff[t] = g.nbr_off[mb + t];
-      bufs.toffT[t] = g.nbr_offT[mb + t];
-      bufs.plist[atomicAdd(bufs.np, 1)] = t;
-    }
-  }
-  for (int w = tid; w < nm * nm; w += nt) {
-    const int dk = w / nm, d2 = w - dk * nm;
-    const bool rowkT = dk == Tr;
-    T u = (T)0;
-    if (d2 >= dk && !(rowkT && d2 >= g.nvn)) u = lu[mrow[dk] + (rowkT ? moffT : moff) + d2];
-    umm[dk * kMaxNodeDofs + d2] = u;
-    if (d2 == dk) rdm[dk] = (T)1 / u;
-  }
-}
-
-template <class T>
-__global__ void __launch_bounds__(256)
-    ilu0_block_kernel(const int *__restrict__ nodes, IluArgs g, const double *__restrict__ A,
-                      T *__restrict__ lu) {
-  extern __shared__ __align__(16) unsigned char sm_raw[];
-  int64_t *srow = reinterpret_cast<int64_t *>(sm_raw);          // [maxnb][maxnr] row starts of m
-  T *blk = reinterpret_cast<T *>(srow + (size_t)g.maxnb * g.maxnr);  // [maxnr][lmax]
-  T *lnm = blk + (size_t)g.maxnr * g.lmax;                       // [16][16] L_nm
-  T *umm2 = lnm + kMaxNodeDofs * kMaxNodeDofs;                   // [2][16][16] U_mm
-  T *rdm2 = umm2 + 2 * kMaxNodeDofs * kMaxNodeDofs;              // [2][16] 1 / U_mm diagonal
-  int *snb = reinterpret_cast<int *>(rdm2 + 2 * kMaxNodeDofs);   // [maxnb] neighbours of n
-  int *soff = snb + g.maxnb;                                     // their column offsets
-  int *sndof = soff + g.maxnb;                                   // their unknown counts
-  int *smb = sndof + g.maxnb;        // lower neighbour m: start of its neighbour list
-  int *smnb = smb + g.maxnb;         // its length
-  int *smoff = smnb + g.maxnb;       // m's own block in m's rows (offset, energy-row offset)
-  int *smoffT = smoff + g.maxnb;
-  int *tab = smoffT + g.maxnb;       // [2][4][maxnb] round-A tables, then [2] counters
-  int *s_np = tab + 8 * g.maxnb;
-  auto bufs = [&](int h) {
-    int *b0 = tab + 4 * h * g.maxnb;
-    return IluRoundA{b0, b0 + g.maxnb, b0 + 2 * g.maxnb, b0 + 3 * g.maxnb, s_np + h};
-  };
-  const int n = nodes[blockIdx.x];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int base = g.nbr_ptr[n], nb = g.nbr_ptr[n + 1] - base;
-  const int f0 = g.fu[n], nr = g.fu[n + 1] - f0;
-  const int Tr = g.energy ? g.dim : -1;  // local index of the energy row
-  const int self = g.nbr_self[n];
-  if (tid < 2) s_np[tid] = 0;
-  for (int s2 = tid; s2 < nb; s2 += nt) {
-    const int q = g.nbr_node[base + s2];
-    snb[s2] = q;
-    soff[s2] = g.nbr_off[base + s2];
-    const int fq = g.fu[q];
-    sndof[s2] = g.fu[q + 1] - fq;
-    if (s2 < self) {
-      const int mb = g.nbr_ptr[q];
-      const int ms = g.nbr_self[q];
-      smb[s2] = mb;
-      smnb[s2] = g.nbr_ptr[q + 1] - mb;
-      smoff[s2] = g.nbr_off[mb + ms];
-      smoffT[s2] = g.nbr_offT[mb + ms];
-      for (int dk = 0; dk < g.fu[q + 1] - fq; dk++)
-        srow[(size_t)s2 * g.maxnr + dk] = g.rowptr[fq + dk];
-    }
-  }
-  __syncthreads();
-  const int L = soff[nb - 1] + sndof[nb - 1];
-  // load the block row (full layout; energy-row pressure columns held at 0)
-  for (int c = tid; c < L; c += nt) {
-    int lo = 0, hi = nb - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (soff[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const int d = c - soff[lo];
-    for (int r = 0; r < nr; r++) {
-      if (r == Tr) {
-        blk[r * g.lmax + c] = d >= g.nvn ? (T)0 : (T)A[g.rowptr[f0 + r] + g.nbr_offT[base + lo] + d];
-      } else {
-        blk[r * g.lmax + c] = (T)A[g.rowptr[f0 + r] + c];
-      }
-    }
-  }
-  if (self > 0)
-    ilu_round_a<T>(g, tid, nt, snb[0], smb[0], smnb[0], sndof[0], Tr, srow, smoff[0], smoffT[0],
-                   snb, nb, lu, bufs(0), umm2, rdm2);
-  __syncthreads();
-  for (int sm = 0; sm < self; sm++) {
-    const int h = sm & 1;
-    const IluRoundA cur = bufs(h);
-    const T *umm = umm2 + h * kMaxNodeDofs * kMaxNodeDofs;
-    const T *rdm = rdm2 + h * kMaxNodeDofs;
-    const int nm = sndof[sm], cm = soff[sm];
-    const int64_t *mrow = srow + (size_t)sm * g.maxnr;
-    // step 1: L_nm = A_nm U_mm^-1, a warp per row (lane d holds the row's
-    // entry in m's column d): per pivot one shuffle, then every later
-    // column updated at once
-    for (int r = tid >> 5; r < nr; r += nt >> 5) {
-      const int lane = tid & 31;
-      T *br = blk + (size_t)r * g.lmax + cm;
-      T v = lane < nm ? br[lane] : (T)0;
-      for (int dk = 0; dk < nm; dk++) {
-        if (r == Tr && dk >= g.nvn) {  // energy row: no pressure columns
-          if (lane == 0) lnm[r * kMaxNodeDofs + dk] = (T)0;
-          continue;
-        }
-        const T l = __shfl_sync(0xffffffffu, v, dk) * rdm[dk];
-        if (lane == dk) v = l;
-        if (lane == 0) lnm[r * kMaxNodeDofs + dk] = l;
-        if (lane > dk && lane < nm && !(r == Tr && lane >= g.nvn))
-          v -= l * umm[dk * kMaxNodeDofs + lane];  // zero where U_mm has no entry
-      }
-      if (lane < nm) br[lane] = v;
-    }
-    __syncthreads();
-    // round A of the next neighbour, into the other half of the tables
-    // (its counter was reset before the barrier that ended its last use)
-    if (sm + 1 < self)
-      ilu_round_a<T>(g, tid, nt, snb[sm + 1], smb[sm + 1], smnb[sm + 1], sndof[sm + 1], Tr,
-                     srow + (size_t)(sm + 1) * g.maxnr, smoff[sm + 1], smoffT[sm + 1], snb, nb,
-                     lu, bufs(h ^ 1), umm2 + (h ^ 1) * kMaxNodeDofs * kMaxNodeDofs,
-                     rdm2 + (h ^ 1) * kMaxNodeDofs);
-    // step 2: A_nq -= L_nm U_mq, one thread per (shared neighbour, column d)
-    // loading the column of U_mq once and updating every row of n
-    const int np = *cur.np;
-    for (int f = tid; f < np * g.maxnr; f += nt) {
-      const int k = f / g.maxnr, d = f - k * g.maxnr;
-      const int t = cur.plist[k], slot = cur.tslot[t];
-      if (d >= sndof[slot]) continue;
-      const int off = cur.toff[t], offT = cur.toffT[t];
-      T u[kMaxNodeDofs];
-#pragma unroll
-      for (int dk = 0; dk < kMaxNodeDofs; dk++) {
-        u[dk] = (T)0;
-        if (dk < nm && !(dk == Tr && d >= g.nvn)) u[dk] = lu[mrow[dk] + (dk == Tr ? offT : off) + d];
-      }
-      T *col = blk + soff[slot] + d;
-      for (int r = 0; r < nr; r++) {
-        if (r == Tr && d >= g.nvn) continue;
-        T acc = (T)0;
-#pragma unroll
-        for (int dk = 0; dk < kMaxNodeDofs; dk++) {
-          if (dk >= nm) break;
-          if (dk == Tr && d >= g.nvn) continue;
-          acc += lnm[r * kMaxNodeDofs + dk] * u[dk];
-        }
-        col[(size_t)r * g.lmax] -= acc;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) *cur.np = 0;  // free for the round A of neighbour sm + 2
-  }
-  // own diagonal block and the rest of the row
-  const int cs = soff[self];
-  for (int dk = 0; dk < nr; dk++) {
-    if (tid == 0) {
-      const T p = blk[dk * g.lmax + cs + dk];
-      if (fabs((double)p) < g.tau) {
-        blk[dk * g.lmax + cs + dk] = p < (T)0 ? (T)-g.tau : (T)g.tau;
-        atomicAdd(g.nfix, 1);
-      }
-    }
-    __syncthreads();
-    const T piv = blk[dk * g.lmax + cs + dk];
-    const int c0 = cs + dk + 1;
-    for (int r = dk + 1; r < nr; r++) {
-      if (r == Tr && dk >= g.nvn) continue;
-      const T l = blk[r * g.lmax + cs + dk] / piv;
-      for (int c = c0 + tid; c < L; c += nt) {
-        const T u = blk[dk * g.lmax + c];
-        if (u == (T)0) continue;
-        if (r == Tr) {
-          // energy row: pressure columns are outside the pattern
-          int lo = 0, hi = nb - 1;
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (soff[mid] <= c) lo = mid; else hi = mid - 1;
-          }
-          if (c - soff[lo] >= g.nvn) continue;
-        }
-        blk[r * g.lmax + c] -= l * u;
-      }
-    }
-    __syncthreads();
-    if (tid < nr && tid > dk && !(tid == Tr && dk >= g.nvn))
-      blk[tid * g.lmax + cs + dk] = blk[tid * g.lmax + cs + dk] / piv;
-    __syncthreads();
-  }
-  // write back
-  for (int c = tid; c < L; c += nt) {
-    int lo = 0, hi = nb - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (soff[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const int d = c - soff[lo];
-    for (int r = 0; r < nr; r++) {
-      if (r == Tr) {
-        if (d < g.nvn) lu[g.rowptr[f0 + r] + g.nbr_offT[base + lo] + d] = blk[r * g.lmax + c];
-      } else {
-        lu[g.rowptr[f0 + r] + c] = blk[r * g.lmax + c];
-      }
-    }
-  }
-}
-
 // Triangular solves: the sync-free sweeps by lines of nodes (gb_sweep.cu), or
 // one launch per dependency level (trsv_level_cta_kernel).
 //
@@ -808,7 +515,7 @@ void build_ilu_schedule(const Layout &L, IluSchedule &S) {
 Solver::~Solver() {
   if (prec64) cudaGraphExecDestroy(prec64);
   if (prec32) cudaGraphExecDestroy(prec32);
-  void *p[] = {d_lu, d_lu32, d_binv, d_binv32, d_Z, d_a32, d_diag, d_lo_nodes, d_up_nodes, d_scale, d_work, d_flags,
+  void *p[] = {d_lu, d_lu32, d_binv, d_binv32, d_Z, d_a32, d_diag, d_lo_nodes, d_up_nodes, d_scale, d_work, d_flags, d_done,
                d_sweep_y, d_V, d_V32, d_t, d_w, d_r, d_xs, d_t32, d_w32};
   for (void *q : p)
     if (q) cudaFree(q);
@@ -828,6 +535,34 @@ Solver::~Solver() {
     cudaError_t e_ = (call);                       \
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
+
+// the factorisation's view of the preconditioner layout
+static IluArgs ilu_args(const Solver *S, const Context *C, int *nfix) {
+  const Layout &L = C->L;
+  IluArgs g;
+  g.fu = S->P.fu;
+  g.rowptr = S->P.rowptr;
+  g.nbr_ptr = S->P.nbr_ptr;
+  g.nbr_node = S->P.nbr_node;
+  g.nbr_off = S->P.nbr_off;
+  g.nbr_offT = S->P.nbr_offT;
+  g.nbr_self = S->P.nbr_self;
+  g.nodes = S->d_lo_nodes;
+  g.num_nodes = L.num_nodes;
+  g.dim = L.dim;
+  g.nvn = L.nvn;
+  g.energy = L.energy;
+  g.maxnb = S->maxnb;
+  g.lmax = S->lmax;
+  g.blkmax = S->blkmax;
+  g.maxnr = L.nvn + L.npres;
+  g.tau = S->pivot_tau;
+  g.nfix = nfix;
+  g.done = S->d_done;
+  g.error = (int *)(S->d_flags + 4);
+  g.spin_limit = kSpinLimit;
+  return g;
+}
 
 int Solver::init(Context *c, int krylov) {
   C = c;
@@ -938,22 +673,33 @@ int Solver::init(Context *c, int krylov) {
                    cudaMemcpyHostToDevice), "sched");
   d_fu = c->d_fu;
   if (L.nvn + L.npres > kMaxNodeDofs) return fail("ILU(0) supports at most 16 unknowns per node");
-  maxnb = 0;
-  lmax = 0;
+  maxnb = lmax = blkmax = 0;
   for (int n = 0; n < LP->num_nodes; n++) {
     const int nb = LP->nbr_ptr[n + 1] - LP->nbr_ptr[n];
     maxnb = std::max(maxnb, nb);
     const int q = LP->nbr_node[LP->nbr_ptr[n + 1] - 1];
-    lmax = std::max(lmax, LP->nbr_off[LP->nbr_ptr[n + 1] - 1] + LP->fu[q + 1] - LP->fu[q]);
+    const int len = LP->nbr_off[LP->nbr_ptr[n + 1] - 1] + LP->fu[q + 1] - LP->fu[q];
+    lmax = std::max(lmax, len);
+    blkmax = std::max(blkmax, (LP->fu[n + 1] - LP->fu[n]) * len);
   }
+  blkmax = (blkmax + 3) / 4 * 4;
   {
-    const size_t sm64 = ilu_smem_bytes(sizeof(double), maxnb, L.nvn + L.npres, lmax);
-    const size_t sm32 = ilu_smem_bytes(sizeof(float), maxnb, L.nvn + L.npres, lmax);
-    if (sm64 > 200 * 1024) return fail("ILU(0) block row does not fit in shared memory");
-    GB_CU(cudaFuncSetAttribute(ilu0_block_kernel<double>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm64), "smem");
-    GB_CU(cudaFuncSetAttribute(ilu0_block_kernel<float>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32), "smem");
+    // the block rows of at most 16 unknowns that the factorisation takes on
+    const size_t maxnr = L.nvn + L.npres;
+    const size_t rows = sizeof(int64_t) * maxnb * maxnr + sizeof(double) * (maxnr * lmax + 800) +
+                        sizeof(int) * (15 * (size_t)maxnb + 4);
+    const IluArgs g = ilu_args(this, C, nullptr);
+    if (rows > 200 * 1024 || ilu_smem_bytes(sizeof(double), g) > 227 * 1024)
+      return fail("ILU(0) block row does not fit in shared memory");
+  }
+  GB_CU(cudaMalloc(&d_done, sizeof(int) * (size_t)(LP->num_nodes + 1)), "ILU flags");
+  GB_CU(cudaMalloc(&d_flags, 16 * sizeof(unsigned)), "trsv error word");
+  GB_CU(cudaMemset(d_flags, 0, 16 * sizeof(unsigned)), "trsv error word");
+  GB_CU(cudaStreamSynchronize(0), "trsv error word");
+  {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   GB_CU(cudaMalloc(&d_lu, sizeof(double) * nnz), "ILU factors");
   GB_CU(cudaMalloc(&d_scale, sizeof(double) * N), "scale");
@@ -1076,23 +822,6 @@ int Solver::factor(const double *vals, bool fp32, cudaStream_t st) {
   d_A = vals;
   int *nfix = (int *)(d_work + kRedBlocks * 3 + 10);
   GB_CU(cudaMemsetAsync(nfix, 0, sizeof(int), st), "pivot count");
-  const Layout &L = C->L;
-  IluArgs g;
-  g.fu = P.fu;
-  g.rowptr = P.rowptr;
-  g.nbr_ptr = P.nbr_ptr;
-  g.nbr_node = P.nbr_node;
-  g.nbr_off = P.nbr_off;
-  g.nbr_offT = P.nbr_offT;
-  g.nbr_self = P.nbr_self;
-  g.dim = L.dim;
-  g.nvn = L.nvn;
-  g.energy = L.energy;
-  g.maxnb = maxnb;
-  g.lmax = lmax;
-  g.maxnr = L.nvn + L.npres;
-  g.tau = pivot_tau;
-  g.nfix = nfix;
   if (fp32 && !d_lu32) {
     GB_CU(cudaMalloc(&d_lu32, sizeof(float) * nnz), "ILU32");
     GB_CU(cudaMalloc(&d_a32, sizeof(float) * nnz), "A32");
@@ -1110,16 +839,10 @@ int Solver::factor(const double *vals, bool fp32, cudaStream_t st) {
     GB_CU(cudaGetLastError(), "matrix permutation");
     Af = d_Ap;
   }
-  for (size_t l = 0; l + 1 < lo_ptr.size(); l++) {
-    const int cnt = lo_ptr[l + 1] - lo_ptr[l];
-    if (fp32) {
-      const size_t sm = ilu_smem_bytes(sizeof(float), maxnb, g.maxnr, lmax);
-      ilu0_block_kernel<float><<<cnt, 256, sm, st>>>(d_lo_nodes + lo_ptr[l], g, Af, d_lu32);
-    } else {
-      const size_t sm = ilu_smem_bytes(sizeof(double), maxnb, g.maxnr, lmax);
-      ilu0_block_kernel<double><<<cnt, 256, sm, st>>>(d_lo_nodes + lo_ptr[l], g, Af, d_lu);
-    }
-  }
+  const IluArgs g = ilu_args(this, C, nfix);
+  GB_CU(cudaMemsetAsync(d_done, 0, sizeof(int) * (size_t)(C->L.num_nodes + 1), st), "ILU flags");
+  GB_CU(fp32 ? ilu0_factor<float>(g, Af, d_lu32, num_sms, st)
+             : ilu0_factor<double>(g, Af, d_lu, num_sms, st), "ILU(0) factorisation");
   GB_CU(cudaGetLastError(), "ILU(0) factorisation");
   {
     const TrsvArgs a = trsv_args(this);
@@ -1154,6 +877,7 @@ int Solver::copy_factors(double *host, bool fp32, cudaStream_t st) {
   const int64_t nnz = C->L.nnz;
   if (ordering != 0) return fail("the factors are in the multicoloured order");
   GB_CU(cudaStreamSynchronize(st), "factor");
+  if (check_trsv_error()) return -1;
   if (fp32) {
     std::vector<float> tmp((size_t)nnz);
     GB_CU(cudaMemcpy(tmp.data(), d_lu32, sizeof(float) * nnz, cudaMemcpyDeviceToHost),
@@ -1167,14 +891,8 @@ int Solver::copy_factors(double *host, bool fp32, cudaStream_t st) {
 
 template <class T>
 static int sync_free_apply(Solver *S, T *z, cudaStream_t st) {
-  if (!S->d_flags) {
-    GB_CU(cudaMalloc(&S->d_flags, 16 * sizeof(unsigned)), "trsv error word");
-    GB_CU(cudaMemsetAsync(S->d_flags, 0, 16 * sizeof(unsigned), st), "trsv error word");
+  if (!S->d_sweep_y)
     GB_CU(cudaMalloc(&S->d_sweep_y, sizeof(double) * (size_t)S->N), "trsv scratch");
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&S->num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
   T *y = static_cast<T *>(S->d_sweep_y);
   LineArgs a{};
   a.error = (int *)(S->d_flags + 4);
@@ -1208,11 +926,12 @@ bool Solver::use_level_graph() const {
 }
 
 int Solver::check_trsv_error() {
-  if (!d_flags) return 0;
   int h = 0;
   GB_CU(cudaMemcpy(&h, d_flags + 4, sizeof(int), cudaMemcpyDeviceToHost), "trsv error");
   if (h) {
-    cudaMemset(d_flags + 4, 0, sizeof(int));
+    GB_CU(cudaMemset(d_flags + 4, 0, sizeof(int)), "trsv error");
+    GB_CU(cudaStreamSynchronize(0), "trsv error");
+    have_lu64 = have_lu32 = false;  // the factors may be what went wrong
     return fail("triangular solve: a dependency wait gave up");
   }
   return 0;

@@ -82,7 +82,9 @@ struct Solver {
   std::vector<int> lo_ptr, up_ptr;
   const double *d_A = nullptr;  // scaled FP64 matrix the factors were built from
   double pivot_tau = 1e-4;      // ILU(0) pivot floor on the row-scaled matrix
-  int maxnb = 0, lmax = 0;      // largest node neighbourhood / block-row length
+  // largest node neighbourhood, row length and block row (values)
+  int maxnb = 0, lmax = 0, blkmax = 0;
+  int *d_done = nullptr;        // nodes whose factors are final (and the next node to draw)
   double *d_scale = nullptr;
   double *d_work = nullptr;     // reduction scratch
   double *h_work = nullptr;     // pinned host mirror
@@ -93,7 +95,7 @@ struct Solver {
   float *d_t32 = nullptr, *d_w32 = nullptr;
   double *d_Z = nullptr;        // m x N preconditioned vectors (flexible GMRES)
   cudaGraphExec_t prec64 = nullptr, prec32 = nullptr;  // captured ILU solves on d_t / d_t32
-  unsigned *d_flags = nullptr;  // sync-free sweeps: [4] error word
+  unsigned *d_flags = nullptr;  // [4] error word, [8] next line to draw (sync-free sweeps)
   void *d_sweep_y = nullptr;    // sync-free sweeps: the L sweep's output (N values)
   int num_sms = 0;
   int check_trsv_error();
