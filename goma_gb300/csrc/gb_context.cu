@@ -126,6 +126,10 @@ Context::~Context() {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (d_sf) cudaFree(d_sf);
+  if (d_s2) cudaFree(d_s2);
+  if (d_ne_ptr) cudaFree(d_ne_ptr);
+  if (d_ne_list) cudaFree(d_ne_list);
+  if (pool) cudaMemPoolDestroy(pool);
   if (ev_k0) cudaEventDestroy(ev_k0);
   if (ev_k1) cudaEventDestroy(ev_k1);
   if (stream) cudaStreamDestroy(stream);
@@ -200,6 +204,31 @@ int Context::init(const gb_problem_desc *d) {
       upload(&d_tab_dphi, tdphi, "tab") || upload(&d_tab_w, tw, "tab") ||
       upload(&d_tab_pt, tpt, "tab") || upload(&d_color_elems, L.color_elems, "colors"))
     return -1;
+  {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (L.dim == 2) {
+      double ell[9], dell[9];
+      for (int a = 0; a < 3; a++)
+        for (int g = 0; g < 3; g++) {
+          ell[a * 3 + g] = lag(a, kPt[g]);
+          dell[a * 3 + g] = dlag(a, kPt[g]);
+        }
+      std::vector<S2Tables> t(1);
+      build_s2_tables(tphi.data(), tdphi.data(), tw.data(), kPt, kLoc9, ell, dell, t[0]);
+      if (upload(&d_s2, t, "tab") || upload(&d_ne_ptr, L.ne_ptr, "node elements") ||
+          upload(&d_ne_list, L.ne_list, "node elements"))
+        return -1;
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return cuda_fail(e, "pool");
+      unsigned long long keep = ~0ull;  // kept for the next assembly, freed with the context
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+  }
   if (L.dim == 3) {
     std::vector<double> iso(112 * 28);
     build_iso_table(tphi.data(), tdphi.data(), iso.data());
@@ -286,19 +315,32 @@ AsmArgs Context::args(const double *x, double *R, double *vals) const {
 
 int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st) {
   if (!st) st = stream;
-  cudaError_t e = cudaMemsetAsync(R, 0, sizeof(double) * L.N, st);
-  if (e == cudaSuccess && vals) e = cudaMemsetAsync(vals, 0, sizeof(double) * L.nnz, st);
-  if (e != cudaSuccess) return cuda_fail(e, "assembly zeroing");
+  cudaError_t e;
   AsmArgs a = args(x, R, vals);
   const int ncol = (int)L.color_ptr.size() - 1;
-  if (timing) cudaEventRecord(ev_k0, st);
-  const int kp = kernel_path(vals != nullptr);
-  if (kp >= 2 && tc_grid == 0) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    tc_grid = 2 * sms;
+  int kp = kernel_path(vals != nullptr);
+  double *blocks = nullptr;  // element blocks of the 2-D path
+  if (kp == 5) {
+    const size_t bytes = sizeof(double) * s2_scratch_values(L.energy != 0, vals != nullptr) *
+                         (size_t)L.num_elems;
+    if (cudaMallocFromPoolAsync((void **)&blocks, bytes, pool, st) != cudaSuccess) {
+      cudaGetLastError();  // no room for the blocks: the scalar kernel
+      kp = 1;
+    }
   }
+  if (timing) cudaEventRecord(ev_k0, st);
+  if (kp == 5) {  // writes every entry of R and vals
+    const S2Nodes nd{L.num_nodes, d_ne_ptr, d_ne_list, L.blkmax};
+    e = launch_assemble_2d(a, L.energy != 0, carreau, vals != nullptr, d_s2, L.num_elems, nd,
+                           blocks, num_sms, st);
+    if (e == cudaSuccess) e = cudaFreeAsync(blocks, st);
+    if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
+  } else {
+    e = cudaMemsetAsync(R, 0, sizeof(double) * L.N, st);
+    if (e == cudaSuccess && vals) e = cudaMemsetAsync(vals, 0, sizeof(double) * L.nnz, st);
+    if (e != cudaSuccess) return cuda_fail(e, "assembly zeroing");
+  }
+  if (kp >= 2) tc_grid = 2 * num_sms;
   for (int c = 0; c < ncol; c++) {
     const int n = L.color_ptr[c + 1] - L.color_ptr[c];
     if (kp == 4)
@@ -310,7 +352,7 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
     else if (kp == 2)
       e = launch_assemble_tc(a, L.energy != 0, carreau, d_color_elems + L.color_ptr[c], n,
                              tc_grid, st);
-    else
+    else if (kp == 1)
       e = launch_assemble(a, L.dim, L.energy != 0, carreau, vals != nullptr,
                           d_color_elems + L.color_ptr[c], n, st);
     if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
@@ -331,13 +373,14 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev_k0, ev_k1);
     kernel_ms += ms;
-    kernel_launches += ncol * (L.nspec > 0 ? 2 : 1);
+    kernel_launches += (kp == 5 ? 2 : ncol) + (L.nspec > 0 ? ncol : 0);
   }
   return 0;
 }
 
 int Context::kernel_path(bool jacobian) const {
-  if (L.dim != 3) return 1;
+  // the 2-D rows are built in shared memory (four nodes a block)
+  if (L.dim != 3) return path == 1 || sizeof(double) * 4 * (size_t)L.blkmax > 200 * 1024 ? 1 : 5;
   // a heat source: the scalar kernel
   if (mat.hsm != GB_HEAT_SOURCE_NONE) return 1;
   const bool gemm_ok = !carreau && mat.viscosity > 0.0;

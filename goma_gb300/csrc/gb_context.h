@@ -24,7 +24,8 @@ struct Context {
   bool carreau = false;
   // element kernel: 0 automatic (4 where it applies, else 1), 1 scalar FP64,
   // 2 DMMA with per-fragment coefficients, 3 DMMA products over operand tables
-  // (3-D Newtonian), 4 sum factorisation (3-D Newtonian)
+  // (3-D Newtonian), 4 sum factorisation (3-D Newtonian); 2-D elements: 1
+  // scalar FP64, any other element blocks and gathered rows
   int path = 0;
   int tc_grid = 0;     // persistent grid of the DMMA kernels
   // ILU triangular solves: 0 sync-free sweeps, 1 level-scheduled graph,
@@ -48,6 +49,13 @@ struct Context {
   double *d_tab_iso = nullptr;  // 3-D: [value, d/dxi_r] x points x nodes (gemm kernel)
   SfTables *d_sf = nullptr;     // 3-D: tables of the sum-factorised kernel
   int *d_color_elems = nullptr;
+  // 2-D: tables and elements of every node; the pool that the element blocks
+  // of an assembly in progress come from (stream-ordered, so that assemblies
+  // on several streams, or captured ones, each have their own)
+  S2Tables *d_s2 = nullptr;
+  int *d_ne_ptr = nullptr, *d_ne_list = nullptr;
+  cudaMemPool_t pool = nullptr;
+  int num_sms = 0;
   double *d_x = nullptr, *d_R = nullptr, *d_vals = nullptr;
   int *d_status = nullptr;
   double *d_elem_rho = nullptr;  // per-element density (gb_set_element_density); NULL: none

@@ -98,6 +98,40 @@ void build_sf_tables(const double *tab_phi, const double *tab_dphi, const int (*
 cudaError_t launch_assemble_sf(const AsmArgs &a, bool energy, const SfTables *tb,
                                const int *elems, int nelem, int grid_cap, cudaStream_t st);
 size_t assemble_sf_smem_bytes();
+// 2-D assembly (gb_assemble_2d.cu): constant tables (1-D Lagrange factors at
+// the Gauss points and their pair products, phi and reference gradients in
+// lexicographic node order, node maps, the upper triangle's rows and columns),
+// the elements of every node, and the element blocks on their way into the
+// matrix: K [element][81 node pairs][fields][fields], P [element][9][2][3]
+// pressure couplings, R [element][9][fields], Rc [element][3].
+struct S2Tables {
+  double ell[2][3][3];
+  double pp[2][9][3];
+  double pu[6][3];  // the distinct l_a l_b, numbered by sym
+  double phi[9][9];
+  double dref[9][9][2];
+  double w[9];
+  double pt[3];
+  int lex[9];
+  int loc[9];
+  int sym[9];
+  uint16_t hmap[18 * 19 / 2];
+};
+struct S2Nodes {
+  int num_nodes;
+  const int *ne_ptr, *ne_list;  // per node: 9 element + local node, ascending
+  int blkmax;                   // most values in the rows of one node
+};
+struct S2Scratch {
+  double *K, *P, *R, *Rc;
+};
+void build_s2_tables(const double *tab_phi, const double *tab_dphi, const double *tab_w,
+                     const double *pt, const int (*loc9)[2], const double *ell,
+                     const double *dell, S2Tables &T);
+size_t s2_scratch_values(bool energy, bool jac);  // per element
+cudaError_t launch_assemble_2d(const AsmArgs &a, bool energy, bool carreau, bool jac,
+                               const S2Tables *tb, int nelem, const S2Nodes &nd, double *scratch,
+                               int sms, cudaStream_t st);
 // 3-D Newtonian residual + Jacobian as dense DMMA products (gb_assemble_gemm.cu);
 // tab_iso is build_iso_table's [112][28] table on the device
 cudaError_t launch_assemble_gemm(const AsmArgs &a, bool energy, const double *tab_iso,

@@ -173,6 +173,18 @@ int build_layout(const gb_problem_desc *d, Layout &L, std::string &err) {
       }
     }
   }
+  if (L.dim == 2) {
+    L.ne_ptr = ne_ptr;
+    L.ne_list.resize(ne_list.size());
+    std::vector<int> fill(nnod, 0);
+    for (int e = 0; e < ne; e++)
+      for (int k = 0; k < nn; k++) {
+        const int n = d->conn[(int64_t)e * nn + k];
+        L.ne_list[ne_ptr[n] + fill[n]++] = e * nn + k;
+      }
+    for (int n = 0; n < nnod; n++)
+      L.blkmax = std::max(L.blkmax, (int)(L.rowptr[L.fu[n + 1]] - L.rowptr[L.fu[n]]));
+  }
   // Dirichlet cards in order, later cards win (src/mm_bc.c:132)
   L.dbc.assign(L.N, 0);
   L.dbc_val.assign(L.N, 0.0);

@@ -26,6 +26,10 @@ struct Layout {
   // For element e and local nodes k, l: index s of node conn[e][l] in the
   // neighbour list of node conn[e][k].
   std::vector<uint16_t> elem_nslot;
+  // 2-D: the elements of every node (9 element + local node, ascending), and
+  // the most matrix entries in the rows of one node
+  std::vector<int> ne_ptr, ne_list;
+  int blkmax = 0;
   std::vector<uint8_t> dbc;     // 1 on Dirichlet / pressure-datum unknowns
   std::vector<double> dbc_val;  // their values (later cards win)
   std::vector<int> color_ptr, color_elems;

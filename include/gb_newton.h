@@ -134,7 +134,9 @@ void *gb_stream(gb_ctx *ctx);
  * residual + Jacobian as DMMA products over shared-memory operand tables,
  * 4 = the 3-D residual + Jacobian by sum factorisation over the
  * tensor-product basis (the fewest FP64 operations).  Paths 3 and 4 take
- * Newtonian viscosity; Carreau and 2-D elements use path 1.  A residual-only
+ * Newtonian viscosity; 3-D Carreau elements use path 1.  2-D elements use
+ * path 1 when it is set and otherwise element blocks by sum factorisation
+ * with every row gathered from its elements.  A residual-only
  * assembly uses the same kernel as the full one under paths 0, 1, 3 and 4,
  * so its R is bitwise the full assembly's; under path 2 it uses path 1.  All
  * give the same matrix to rounding. */
