@@ -357,8 +357,11 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
                           d_color_elems + L.color_ptr[c], n, st);
     if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
     if (L.nspec > 0) {
-      e = launch_assemble_species(a, L.dim, L.energy != 0, vals != nullptr,
-                                  d_color_elems + L.color_ptr[c], n, st);
+      e = L.dim == 3 && path != 1
+              ? launch_assemble_species_sf(a, L.energy != 0, vals != nullptr, d_sf,
+                                           d_color_elems + L.color_ptr[c], n, num_sms, st)
+              : launch_assemble_species(a, L.dim, L.energy != 0, vals != nullptr,
+                                        d_color_elems + L.color_ptr[c], n, st);
       if (e != cudaSuccess) return cuda_fail(e, "species assembly launch");
     }
   }

@@ -93,6 +93,10 @@ struct SfTables {
   int loc[27];
   uint16_t hmap[81 * 82 / 2];
 };
+// species rows of 3-D elements by sum factorisation (gb_assemble_species.cu)
+cudaError_t launch_assemble_species_sf(const AsmArgs &a, bool energy, bool jac,
+                                       const SfTables *tb, const int *elems, int nelem, int sms,
+                                       cudaStream_t st);
 void build_sf_tables(const double *tab_phi, const double *tab_dphi, const int (*loc27)[3],
                      const double *ell, const double *dell, SfTables &T);
 cudaError_t launch_assemble_sf(const AsmArgs &a, bool energy, const SfTables *tb,

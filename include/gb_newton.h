@@ -136,7 +136,8 @@ void *gb_stream(gb_ctx *ctx);
  * tensor-product basis (the fewest FP64 operations).  Paths 3 and 4 take
  * Newtonian viscosity; 3-D Carreau elements use path 1.  2-D elements use
  * path 1 when it is set and otherwise element blocks by sum factorisation
- * with every row gathered from its elements.  A residual-only
+ * with every row gathered from its elements; species rows of 3-D elements
+ * are summed by factors too unless path 1 is set.  A residual-only
  * assembly uses the same kernel as the full one under paths 0, 1, 3 and 4,
  * so its R is bitwise the full assembly's; under path 2 it uses path 1.  All
  * give the same matrix to rounding. */
