@@ -22,26 +22,37 @@
 //     weights (-rho dA dv_a/dx_b, -rho Cp dA dT/dx_b, dA) and the advection
 //     term S1(i,j) = sum_q phi_i (-rho dA v . grad phi_j) written as three
 //     such sums over reference derivatives: phi_i phi_j = prod_d
-//     l_{i_d}(q_d) l_{j_d}(q_d), so each is three contractions of 243 + 729
-//     + 2187 FMA instead of 19,683;
-//   H((p,i),(r,j)) = sum_q dphi_i/dx_p dA dphi_j/dx_r, symmetric 81 x 81,
-//     upper triangle only (3,321 entries x 27 FMA): gives the transpose
+//     l_{i_d}(q_d) l_{j_d}(q_d), so each is three contractions, and since
+//     l_a l_b has 6 distinct values a direction a mass matrix has 216, 162 +
+//     324 + 648 FMA instead of 19,683 (an advection term 324, ~1,600 FMA);
+//   residual rows: the same way, 729 FMA each instead of 2,916;
+//   H((p,i),(r,j)) = sum_q dphi_i/dx_p dA dphi_j/dx_r: gives the transpose
 //     stress term -mu H((b,i),(a,j)) of J_ab, and through its trace the
-//     viscous term of J_aa and the conduction term of J_TT.
+//     viscous term of J_aa and the conduction term of J_TT.  A thread keeps
+//     the 3 x 3 block of a node pair i <= j in registers (9 FMA from 6 loads)
+//     and forms J(i,j) and J(j,i) from it, 378 x 9 x 27 FMA.
 //
 //   J_ab   = M(-rho dA dv_a/dx_b) - mu H((b,i),(a,j)) + delta_ab (S1 - mu tr H)
 //   J_TT   = Cp S1 - k tr H
 //   J_Tb   = M(-rho Cp dA dT/dx_b),   J_aT = (df_a/dT) M(dA)
 //   J_mP   = sum_q dphi_i/dx_a psi_l dA,   J_cv = J_mP^T
 //
-// That is ~195K FP64 operations per element against ~865K for the dense
-// forms.  The scatter adds into the CSR values with red.global.add.f64: the
-// add runs in L2 instead of on the SM's FP64 pipe, and since the elements of
-// one colour share no CSR row every entry receives one add per launch, so
-// the result is deterministic.  One CTA of 256 threads per element, two
-// CTAs per SM, persistent over the colour's element list.
+// That is ~160K FP64 operations per element against ~865K for the dense
+// forms; at 2 FMA a clock 13,824 elements (24^3) cannot take less than
+// ~3.8 ms.  Measured 4.27 ms, 5.45 ms for 324 products a mass matrix, a dense
+// residual and H entry by entry through shared memory (two loads an FMA).
+//
+// The scatter adds into the CSR values with red.global.add.f64: the add runs
+// in L2 instead of on the SM's FP64 pipe, and since the elements of one
+// colour share no CSR row every entry receives one add per launch, so the
+// result is deterministic.  One CTA of 192 threads per element (378 pairs in
+// two rounds), persistent over the colour's element list.  Stages that
+// follow one another share memory, 71 KB a CTA, so that three of them fill
+// the gaps of each other's serial parts: H, the masses and the operands side
+// by side left room for two (648 us instead of 575 us for 1,728 elements).
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "gb_device.h"
@@ -53,44 +64,57 @@ namespace sf {
 constexpr int NN = 27, NQ = 27, NP = 4, CENT = 20, NF = 7;
 constexpr int NC = 16;  // sum-factorised contractions
 enum { C_AB = 0, C_TV = 9, C_DA = 12, C_S1 = 13 };
-constexpr int NH = 81 * 82 / 2;  // upper triangle of H
-
-__device__ __forceinline__ int hrow(int P) { return P * 81 - (P * (P - 1)) / 2; }
+// Their distinct values: phi_i phi_j = prod_d l_a l_b has 6 factors a
+// direction (l_a l_b is symmetric), the advection term along direction d 9 in
+// that one (l_a l'_b).
+constexpr int SYM = 216, ADV = 324;
+constexpr int NPAIR = 27 * 28 / 2;  // node pairs i <= j
+constexpr int NT = 192;             // threads: two rounds of node pairs
 
 struct Smem {
   double ell[2][3][3];   // [0] l_a(xi_g), [1] l'_a(xi_g)
-  double pp[2][9][3];    // [0] l_a l_b, [1] l_a l'_b at xi_g, index a*3+b
-  double phi[NQ][NN];    // phi_L(q), L lexicographic
-  double W[NC][NQ];      // weights of the sum-factorised contractions
-  double cR[4][NQ];      // residual: phi part (momentum a, energy 3)
-  double tR[3][4][NQ];   // residual: gradient part [p][n][q]
+  double pS[6][3];       // l_a l_b at xi_g, pair number sym[a*3+b]
+  double pLD[9][3];      // l_a l'_b, index a*3+b
   double psidA[NP][NQ];
   double Bq[NQ][9];      // J^-1 [p][r]
   double dAq[NQ];
-  double G[3][NQ][NN];   // d phi_L / d x_p at q
-  double cG[3][NQ][NN];  // dA * G
-  double T2[NC][3][81];  // second stage of the sum factorisation
+  double Mw[13][SYM];    // the contractions' values
+  double S1[3][ADV];
   union {
-    double H[NH];
-    double T1[NC][9][9];
-    struct {
-      double Xn[NF][NN];   // x y z u v w T at the nodes (lexicographic)
+    struct {             // fields at the nodes and, contracted, at the points
       double A[NF][2][NN];
       double B[NF][3][NN];
-      double F[NF][4][NQ]; // value, d/dxi_1..3 at the points
+      double Xn[NF][NN];   // x y z u v w T at the nodes (lexicographic)
       double Xd[4][NN];    // u v w T time derivatives at the nodes (transient)
+      double F[NF][4][NQ]; // value, d/dxi_1..3 at the points
     } iso;
+    struct {
+      double W[NC][NQ];      // weights of the sum-factorised contractions
+      // residual of momentum a and energy 3: phi part, then the parts of the
+      // reference gradients; contracted over the first and second direction
+      double cR[4][4][NQ];
+      double rP[4][3][NQ], rQ[4][2][NQ];
+      double A[NC][81];   // contracted over the third direction [q12][pair]
+      double B[13][3][36], BS[3][3][54];  // and the second [q1][pairs]
+    } st;
+    struct {
+      double G[3][NQ][NN];   // d phi_L / d x_p at q
+      double cG[3][NQ][NN];  // dA * G
+    } g;
   } X;
   double Pn[NP];
+  int sym[9];
   int lex[NN];    // lexicographic index of local node k
   int loc[NN];    // local node of lexicographic index L
   int nodes[NN];  // global node of local node k
 };
+// the points' set-up reads Xn, Xd and F while it writes W and cR
+static_assert(offsetof(Smem, X.iso.Xn) >= offsetof(Smem, X.st.rP), "iso overlaps W, cR");
 
 }  // namespace sf
 
 template <bool ENERGY, bool JAC>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(sf::NT, 3)
     assemble_sf_kernel(AsmArgs A, const SfTables *__restrict__ tb,
                        const int *__restrict__ elems, int nelem) {
   using namespace sf;
@@ -103,8 +127,13 @@ __global__ void __launch_bounds__(256, 2)
 
   // constant tables
   for (int t = tid; t < 18; t += nt) (&S.ell[0][0][0])[t] = (&tb->ell[0][0][0])[t];
-  for (int t = tid; t < 54; t += nt) (&S.pp[0][0][0])[t] = (&tb->pp[0][0][0])[t];
-  for (int t = tid; t < NQ * NN; t += nt) (&S.phi[0][0])[t] = (&tb->phi[0][0])[t];
+  for (int t = tid; t < 27; t += nt) {
+    const int a = t / 9, b = (t / 3) % 3, g = t % 3;
+    const int lo = a < b ? a : b, u = lo * 3 - lo * (lo - 1) / 2 + (a < b ? b - a : a - b);
+    S.pLD[a * 3 + b][g] = tb->pp[1][a * 3 + b][g];
+    if (a <= b) S.pS[u][g] = tb->pp[0][a * 3 + b][g];
+    S.sym[a * 3 + b] = u;
+  }
   for (int t = tid; t < NN; t += nt) {
     S.lex[t] = tb->lex[t];
     S.loc[t] = tb->loc[t];
@@ -221,7 +250,7 @@ __global__ void __launch_bounds__(256, 2)
         double vd[4] = {0.0, 0.0, 0.0, 0.0};
         if (A.xdot)
           for (int L = 0; L < NN; L++) {
-            const double ph = S.phi[q][L];
+            const double ph = __ldg(&tb->phi[q][L]);
 #pragma unroll
             for (int c = 0; c < 4; c++) vd[c] = fma(ph, S.X.iso.Xd[c][L], vd[c]);
           }
@@ -233,25 +262,31 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (int a = 0; a < 3; a++) {
 #pragma unroll
-          for (int b = 0; b < 3; b++) S.W[C_AB + a * 3 + b][q] = -rho * dA * gv[b][a];
-          S.W[C_TV + a][q] = ENERGY ? -rho * M.heat_capacity * dA * gT[a] : 0.0;
-          S.W[C_S1 + a][q] = -rho * dA * (v[0] * B[0][a] + v[1] * B[1][a] + v[2] * B[2][a]);
+          for (int b = 0; b < 3; b++) S.X.st.W[C_AB + a * 3 + b][q] = -rho * dA * gv[b][a];
+          S.X.st.W[C_TV + a][q] = ENERGY ? -rho * M.heat_capacity * dA * gT[a] : 0.0;
+          S.X.st.W[C_S1 + a][q] = -rho * dA * (v[0] * B[0][a] + v[1] * B[1][a] + v[2] * B[2][a]);
           double f = M.source[a];
           if (M.source_model == GB_SOURCE_BOUSSINESQ)
             f = ENERGY ? rho * M.source[a] * (-M.beta * (T - M.Tref)) : 0.0;
           const double adv = v[0] * gv[0][a] + v[1] * gv[1][a] + v[2] * gv[2][a];
           // with the mass term -rho v_dot_a (src/mm_fill_momentum.c:471-500)
-          S.cR[a][q] = dA * (f - rho * (adv + vd[a]));
+          S.X.st.cR[a][0][q] = dA * (f - rho * (adv + vd[a]));
+          double t[3];
 #pragma unroll
           for (int p = 0; p < 3; p++)
-            S.tR[p][a][q] = -dA * ((p == a ? -P : 0.0) + mu * (gv[a][p] + gv[p][a]));
-        }
-        S.W[C_DA][q] = dA;
-        S.cR[3][q] = ENERGY ? -rho * M.heat_capacity * dA *
-                                  (v[0] * gT[0] + v[1] * gT[1] + v[2] * gT[2] + vd[3])
-                            : 0.0;
+            t[p] = -dA * ((p == a ? -P : 0.0) + mu * (gv[a][p] + gv[p][a]));
 #pragma unroll
-        for (int p = 0; p < 3; p++) S.tR[p][3][q] = ENERGY ? -M.conductivity * dA * gT[p] : 0.0;
+          for (int r = 0; r < 3; r++)
+            S.X.st.cR[a][1 + r][q] = B[0][r] * t[0] + B[1][r] * t[1] + B[2][r] * t[2];
+        }
+        S.X.st.W[C_DA][q] = dA;
+        S.X.st.cR[3][0][q] = ENERGY ? -rho * M.heat_capacity * dA *
+                                     (v[0] * gT[0] + v[1] * gT[1] + v[2] * gT[2] + vd[3])
+                               : 0.0;
+        const double kdA = ENERGY ? -M.conductivity * dA : 0.0;
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+          S.X.st.cR[3][1 + r][q] = kdA * (B[0][r] * gT[0] + B[1][r] * gT[1] + B[2][r] * gT[2]);
 #pragma unroll
         for (int p = 0; p < 3; p++)
 #pragma unroll
@@ -276,114 +311,117 @@ __global__ void __launch_bounds__(256, 2)
       }
     }
     __syncthreads();
-    // ---- physical gradients; first stage of the sum factorisation
+    // three contractions over the directions: masses and advection (A, B,
+    // values), residual rows (rP, rQ, rows)
+    constexpr int NRES = ENERGY ? 4 : 3;
+    if (JAC) {
+      for (int t = tid; t < NC * 81; t += nt) {
+        const int c = t / 81, r = t % 81, q12 = r % 9, k3 = r / 9;
+        if (k3 >= (c == C_S1 + 2 ? 9 : 6)) continue;
+        const double *pp = c == C_S1 + 2 ? S.pLD[k3] : S.pS[k3];
+        const double *w = &S.X.st.W[c][q12];
+        S.X.st.A[c][k3 * 9 + q12] = pp[0] * w[0] + pp[1] * w[9] + pp[2] * w[18];
+      }
+    }
+    for (int t = tid; t < NRES * 81; t += nt) {
+      const int n = t / 81, p = (t / 27) % 3, r = t % 27, a1 = r % 3;
+      const double *c = &S.X.st.cR[n][p == 0 ? 0 : 1 + p][r - a1];
+      const double *l = S.ell[0][a1];
+      double v = l[0] * c[0] + l[1] * c[1] + l[2] * c[2];
+      if (p == 0) {
+        const double *g = &S.X.st.cR[n][1][r - a1], *d = S.ell[1][a1];
+        v += d[0] * g[0] + d[1] * g[1] + d[2] * g[2];
+      }
+      S.X.st.rP[n][p][r] = v;
+    }
+    __syncthreads();
+    // ---- second direction; Dirichlet diagonals
+    if (JAC) {
+      for (int t = tid; t < 13 * 108; t += nt) {
+        const int c = t / 108, r = t % 108, q1 = r / 36, k23 = r % 36;
+        const double *pp = S.pS[k23 / 6], *A1 = &S.X.st.A[c][(k23 % 6) * 9 + q1];
+        S.X.st.B[c][q1][k23] = pp[0] * A1[0] + pp[1] * A1[3] + pp[2] * A1[6];
+      }
+      for (int t = tid; t < 3 * 162; t += nt) {
+        const int c = t / 162, r = t % 162, q1 = r / 54, k23 = r % 54;
+        const int n3 = c == 2 ? 9 : 6, k2 = k23 / n3, k3 = k23 - k2 * n3;
+        if (c == 0 && k2 >= 6) continue;
+        const double *pp = c == 1 ? S.pLD[k2] : S.pS[k2];
+        const double *A1 = &S.X.st.A[C_S1 + c][k3 * 9 + q1];
+        S.X.st.BS[c][q1][k23] = pp[0] * A1[0] + pp[1] * A1[3] + pp[2] * A1[6];
+      }
+    }
+    for (int t = tid; t < NRES * 54; t += nt) {
+      const int n = t / 54, p = (t / 27) & 1, r = t % 27, a2 = (r / 3) % 3;
+      const double *c = &S.X.st.rP[n][p ? 2 : 0][r - 3 * a2], *l = S.ell[0][a2];
+      double v = l[0] * c[0] + l[1] * c[3] + l[2] * c[6];
+      if (p == 0) {
+        const double *g = &S.X.st.rP[n][1][r - 3 * a2], *d = S.ell[1][a2];
+        v += d[0] * g[0] + d[1] * g[3] + d[2] * g[6];
+      }
+      S.X.st.rQ[n][p][r] = v;
+    }
+    if (JAC) {
+      for (int t = tid; t < NN * NV + NP; t += nt) {
+        int k, var;
+        if (t < NN * NV) {
+          k = t / NV;
+          var = t - k * NV;
+        } else {
+          k = CENT;
+          var = A.pofs + t - NN * NV;
+        }
+        const int nk = S.nodes[k];
+        const int gr = A.fu[nk] + var;
+        if (!A.dbc[gr]) continue;
+        const int s = A.elem_nslot[(int64_t)e * NN * NN + k * NN + k];
+        const int off = (ENERGY && var == DIM) ? A.nbr_offT[A.nbr_ptr[nk] + s]
+                                               : A.nbr_off[A.nbr_ptr[nk] + s];
+        atomicAdd(A.vals + A.rowptr[gr] + off + var, 1.0);
+      }
+    }
+    __syncthreads();
+    // ---- third direction
+    for (int t = tid; t < NRES * NN; t += nt) {
+      const int n = t / NN, L = t % NN, a3 = L / 9;
+      const double *c = &S.X.st.rQ[n][0][L % 9], *g = &S.X.st.rQ[n][1][L % 9];
+      const double *l = S.ell[0][a3], *d = S.ell[1][a3];
+      const double v = l[0] * c[0] + l[1] * c[9] + l[2] * c[18] + d[0] * g[0] + d[1] * g[9] +
+                       d[2] * g[18];
+      const int gr = A.fu[S.nodes[S.loc[L]]] + n;
+      if (!A.dbc[gr]) atomicAdd(A.R + gr, v);
+    }
+    if constexpr (JAC) {
+    for (int t = tid; t < 13 * SYM; t += nt) {
+      const int c = t / SYM, r = t % SYM, k23 = r % 36;
+      const double *pp = S.pS[r / 36];
+      S.Mw[c][r] = pp[0] * S.X.st.B[c][0][k23] + pp[1] * S.X.st.B[c][1][k23] +
+                   pp[2] * S.X.st.B[c][2][k23];
+    }
+    for (int t = tid; t < 3 * ADV; t += nt) {
+      const int c = t / ADV, r = t % ADV, n23 = c == 0 ? 36 : 54, k1 = r / n23, k23 = r - k1 * n23;
+      const double *pp = c == 0 ? S.pLD[k1] : S.pS[k1];
+      S.S1[c][r] = pp[0] * S.X.st.BS[c][0][k23] + pp[1] * S.X.st.BS[c][1][k23] +
+                   pp[2] * S.X.st.BS[c][2][k23];
+    }
+    __syncthreads();
+    // ---- physical gradients
     for (int t = tid; t < NQ * NN; t += nt) {
       const int q = t / NN, L = t - q * NN;
       const double *d = &tb->dref[q][L][0];
       const double d0 = __ldg(d), d1 = __ldg(d + 1), d2 = __ldg(d + 2);
       const double *B = S.Bq[q];
-      const double g0 = B[0] * d0 + B[1] * d1 + B[2] * d2;
-      const double g1 = B[3] * d0 + B[4] * d1 + B[5] * d2;
-      const double g2 = B[6] * d0 + B[7] * d1 + B[8] * d2;
-      S.G[0][q][L] = g0;
-      S.G[1][q][L] = g1;
-      S.G[2][q][L] = g2;
-      if (JAC) {
-        const double dA = S.dAq[q];
-        S.cG[0][q][L] = dA * g0;
-        S.cG[1][q][L] = dA * g1;
-        S.cG[2][q][L] = dA * g2;
-      }
-    }
-    if (JAC) {
-      for (int t = tid; t < NC * 81; t += nt) {
-        const int c = t / 81, r = t % 81, q12 = r / 9, ab3 = r % 9;
-        const double *pp = S.pp[c == C_S1 + 2 ? 1 : 0][ab3];
-        const double *w = &S.W[c][q12];
-        S.X.T1[c][q12][ab3] = pp[0] * w[0] + pp[1] * w[9] + pp[2] * w[18];
-      }
-    }
-    __syncthreads();
-    // ---- second stage; residual rows, J_mP / J_cv, Dirichlet diagonals
-    if (JAC) {
-      for (int t = tid; t < NC * 243; t += nt) {
-        const int c = t / 243, r = t % 243, q1 = r / 81, ab23 = r % 81;
-        const int ab2 = ab23 / 9, ab3 = ab23 % 9;
-        const double *pp = S.pp[c == C_S1 + 1 ? 1 : 0][ab2];
-        S.T2[c][q1][ab23] = pp[0] * S.X.T1[c][q1][ab3] + pp[1] * S.X.T1[c][q1 + 3][ab3] +
-                            pp[2] * S.X.T1[c][q1 + 6][ab3];
-      }
-    }
-    {
-      const int nres = 4 * NN, njmp = JAC ? 3 * NN * NP : 0, ndir = JAC ? NN * NV + NP : 0;
-      const int nc = S.nodes[CENT];
-      for (int t = tid; t < nres + njmp + ndir; t += nt) {
-        if (t < nres) {
-          const int n = t / NN, L = t % NN;
-          if (n == 3 && !ENERGY) continue;
-          double s = 0.0;
-#pragma unroll 3
-          for (int q = 0; q < NQ; q++) {
-            s = fma(S.phi[q][L], S.cR[n][q], s);
-            s = fma(S.G[0][q][L], S.tR[0][n][q], s);
-            s = fma(S.G[1][q][L], S.tR[1][n][q], s);
-            s = fma(S.G[2][q][L], S.tR[2][n][q], s);
-          }
-          const int gr = A.fu[S.nodes[S.loc[L]]] + n;
-          if (!A.dbc[gr]) atomicAdd(A.R + gr, s);
-        } else if (t < nres + njmp) {
-          const int u = t - nres, a = u / (NN * NP), L = (u / NP) % NN, l = u % NP;
-          double s = 0.0;
-#pragma unroll 3
-          for (int q = 0; q < NQ; q++) s = fma(S.G[a][q][L], S.psidA[l][q], s);
-          const int k = S.loc[L], nk = S.nodes[k];
-          const uint16_t *ns = A.elem_nslot + (int64_t)e * NN * NN;
-          const int gr = A.fu[nk] + a;
-          if (!A.dbc[gr])
-            atomicAdd(A.vals + A.rowptr[gr] + A.nbr_off[A.nbr_ptr[nk] + ns[k * NN + CENT]] +
-                          A.pofs + l, s);
-          const int gc = A.fu[nc] + A.pofs + l;
-          if (!A.dbc[gc])
-            atomicAdd(A.vals + A.rowptr[gc] + A.nbr_off[A.nbr_ptr[nc] + ns[CENT * NN + k]] + a, s);
-        } else {
-          const int u = t - nres - njmp;
-          int k, var;
-          if (u < NN * NV) {
-            k = u / NV;
-            var = u - k * NV;
-          } else {
-            k = CENT;
-            var = A.pofs + u - NN * NV;
-          }
-          const int nk = S.nodes[k];
-          const int gr = A.fu[nk] + var;
-          if (!A.dbc[gr]) continue;
-          const int s = A.elem_nslot[(int64_t)e * NN * NN + k * NN + k];
-          const int off = (ENERGY && var == DIM) ? A.nbr_offT[A.nbr_ptr[nk] + s]
-                                                 : A.nbr_off[A.nbr_ptr[nk] + s];
-          atomicAdd(A.vals + A.rowptr[gr] + off + var, 1.0);
-        }
-      }
-    }
-    if (!JAC) continue;
-    __syncthreads();
-    // ---- H, upper triangle
-    for (int t = tid; t < NH; t += nt) {
-      const int pr = tb->hmap[t];
-      const int P = pr >> 7, R = pr & 127;
-      const int p = P / NN, i = P - p * NN, r = R / NN, j = R - r * NN;
-      const double *gi = &S.G[p][0][i], *gj = &S.cG[r][0][j];
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+      const double dA = S.dAq[q];
 #pragma unroll
-      for (int q = 0; q < NQ; q += 3) {
-        s0 = fma(gi[q * NN], gj[q * NN], s0);
-        s1 = fma(gi[(q + 1) * NN], gj[(q + 1) * NN], s1);
-        s2 = fma(gi[(q + 2) * NN], gj[(q + 2) * NN], s2);
+      for (int p = 0; p < 3; p++) {
+        const double g = B[3 * p] * d0 + B[3 * p + 1] * d1 + B[3 * p + 2] * d2;
+        S.X.g.G[p][q][L] = g;
+        S.X.g.cG[p][q][L] = dA * g;
       }
-      S.X.H[t] = (s0 + s1) + s2;
     }
     __syncthreads();
-    // ---- node pairs: combine and scatter
+    // ---- node pairs (i, j), i <= j: the 3 x 3 block of H in registers, then
+    // J(i, j) and J(j, i)
     {
       const double mu = M.viscosity, Cp = M.heat_capacity, kc = M.conductivity;
       double dfT[3];
@@ -393,53 +431,100 @@ __global__ void __launch_bounds__(256, 2)
                      ? -rho_e * M.source[a] * M.beta
                      : 0.0;
       const uint16_t *ns = A.elem_nslot + (int64_t)e * NN * NN;
-      for (int t = tid; t < NN * NN; t += nt) {
-        const int ki = t / NN, kj = t - ki * NN;
-        const int Li = S.lex[ki], Lj = S.lex[kj];
+      const bool tr = A.mass_c != 0.0;
+      for (int t = tid; t < NPAIR; t += nt) {
+        const int pr = tb->pmap[t];
+        const int Li = pr >> 5, Lj = pr & 31;
+        double h[3][3];  // H((p, i), (r, j))
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+#pragma unroll
+          for (int r = 0; r < 3; r++) h[p][r] = 0.0;
+        const double *gi = &S.X.g.G[0][0][Li], *gj = &S.X.g.cG[0][0][Lj];
+#pragma unroll 9
+        for (int q = 0; q < NQ; q++) {
+          double u[3], w[3];
+#pragma unroll
+          for (int p = 0; p < 3; p++) {
+            u[p] = gi[(p * NQ + q) * NN];
+            w[p] = gj[(p * NQ + q) * NN];
+          }
+#pragma unroll
+          for (int p = 0; p < 3; p++)
+#pragma unroll
+            for (int r = 0; r < 3; r++) h[p][r] = fma(u[p], w[r], h[p][r]);
+        }
         const int a1 = Li % 3, a2 = (Li / 3) % 3, a3 = Li / 9;
         const int b1 = Lj % 3, b2 = (Lj / 3) % 3, b3 = Lj / 9;
-        const int ab1 = a1 * 3 + b1, ab23 = (a2 * 3 + b2) * 9 + a3 * 3 + b3;
-        auto stage3 = [&](int c) {
-          const double *pp = S.pp[c == C_S1 ? 1 : 0][ab1];
-          return pp[0] * S.T2[c][0][ab23] + pp[1] * S.T2[c][1][ab23] + pp[2] * S.T2[c][2][ab23];
-        };
-        auto h = [&](int P, int R) {
-          return P <= R ? S.X.H[hrow(P) + R - P] : S.X.H[hrow(R) + P - R];
-        };
-        const double S1 = stage3(C_S1) + stage3(C_S1 + 1) + stage3(C_S1 + 2);
-        const double trH = h(Li, Lj) + h(NN + Li, NN + Lj) + h(2 * NN + Li, 2 * NN + Lj);
-        const int ni = S.nodes[ki];
-        const int fi = A.fu[ni];
-        const int nb = A.nbr_ptr[ni] + ns[ki * NN + kj];
-        const bool tr = A.mass_c != 0.0;
-        const double mdA = (ENERGY || tr) ? stage3(C_DA) : 0.0;
+        const int s1 = S.sym[a1 * 3 + b1], s2 = S.sym[a2 * 3 + b2], s3 = S.sym[a3 * 3 + b3];
+        const int m = (s1 * 6 + s2) * 6 + s3;
+        const double trH = h[0][0] + h[1][1] + h[2][2];
+        const double mdA = (ENERGY || tr) ? S.Mw[C_DA][m] : 0.0;
         // the mass terms' sensitivity -(1 + 2 theta) / dt rho M(dA)
         // (src/mm_fill_momentum.c:1586-1590), times Cp on the energy row
         const double Mt = tr ? -A.mass_c * rho_e * mdA : 0.0;
-        const double D = fma(-mu, trH, S1) + Mt;
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-          const int gr = fi + a;
-          if (A.dbc[gr]) continue;
-          double *row = A.vals + A.rowptr[gr] + A.nbr_off[nb];
+        for (int p = 0; p < 3; p++)
 #pragma unroll
-          for (int b = 0; b < 3; b++) {
-            double v = fma(-mu, h(b * NN + Li, a * NN + Lj), stage3(C_AB + a * 3 + b));
-            if (a == b) v += D;
-            atomicAdd(row + b, v);
+          for (int r = 0; r < 3; r++) h[p][r] *= -mu;
+#pragma unroll 1
+        for (int o = 0; o < (Li == Lj ? 1 : 2); o++) {  // rows of i, then of j
+          const int ki = S.loc[o ? Lj : Li], kj = S.loc[o ? Li : Lj];
+          const int f1 = o ? b1 * 3 + a1 : a1 * 3 + b1, f2 = o ? b2 * 3 + a2 : a2 * 3 + b2,
+                    f3 = o ? b3 * 3 + a3 : a3 * 3 + b3;
+          const double S1 = S.S1[0][(f1 * 6 + s2) * 6 + s3] + S.S1[1][(s1 * 9 + f2) * 6 + s3] +
+                            S.S1[2][(s1 * 6 + s2) * 9 + f3];
+          const double D = fma(-mu, trH, S1) + Mt;
+          const int ni = S.nodes[ki];
+          const int fi = A.fu[ni];
+          const int nb = A.nbr_ptr[ni] + ns[ki * NN + kj];
+          const int off = A.nbr_off[nb];
+#pragma unroll
+          for (int a = 0; a < 3; a++) {
+            const int gr = fi + a;
+            if (A.dbc[gr]) continue;
+            double *row = A.vals + A.rowptr[gr] + off;
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+              double v = (o ? h[a][b] : h[b][a]) + S.Mw[C_AB + a * 3 + b][m];
+              if (a == b) v += D;
+              atomicAdd(row + b, v);
+            }
+            if (ENERGY) atomicAdd(row + DIM, dfT[a] * mdA);
           }
-          if (ENERGY) atomicAdd(row + DIM, dfT[a] * mdA);
-        }
-        if (ENERGY) {
-          const int gr = fi + DIM;
-          if (!A.dbc[gr]) {
-            double *row = A.vals + A.rowptr[gr] + A.nbr_offT[nb];
+          if (ENERGY) {
+            const int gr = fi + DIM;
+            if (!A.dbc[gr]) {
+              double *row = A.vals + A.rowptr[gr] + A.nbr_offT[nb];
 #pragma unroll
-            for (int b = 0; b < 3; b++) atomicAdd(row + b, stage3(C_TV + b));
-            atomicAdd(row + DIM, fma(Cp, S1 + Mt, -kc * trH));
+              for (int b = 0; b < 3; b++) atomicAdd(row + b, S.Mw[C_TV + b][m]);
+              atomicAdd(row + DIM, fma(Cp, S1 + Mt, -kc * trH));
+            }
           }
         }
       }
+      // ---- J_mP / J_cv: two pressure modes of one (a, node)
+      for (int t = tid; t < 3 * NN * 2; t += nt) {
+        const int a = t / (NN * 2), L = (t >> 1) % NN, l0 = (t & 1) * 2;
+        double s[2] = {0.0, 0.0};
+#pragma unroll 9
+        for (int q = 0; q < NQ; q++) {
+          const double g = S.X.g.G[a][q][L];
+          s[0] = fma(g, S.psidA[l0][q], s[0]);
+          s[1] = fma(g, S.psidA[l0 + 1][q], s[1]);
+        }
+        const int k = S.loc[L], nk = S.nodes[k], nc = S.nodes[CENT];
+        const int gr = A.fu[nk] + a, gc = A.fu[nc] + A.pofs + l0;
+        double *row = A.vals + A.rowptr[gr] + A.nbr_off[A.nbr_ptr[nk] + ns[k * NN + CENT]] +
+                      A.pofs + l0;
+        const int oc = A.nbr_off[A.nbr_ptr[nc] + ns[CENT * NN + k]] + a;
+#pragma unroll
+        for (int l = 0; l < 2; l++) {
+          if (!A.dbc[gr]) atomicAdd(row + l, s[l]);
+          if (!A.dbc[gc + l]) atomicAdd(A.vals + A.rowptr[gc + l] + oc, s[l]);
+        }
+      }
+    }
     }
   }
 }
@@ -470,8 +555,8 @@ void build_sf_tables(const double *tab_phi, const double *tab_dphi, const int (*
       for (int r = 0; r < 3; r++) T.dref[q][L][r] = tab_dphi[(q * NN + k) * 3 + r];
     }
   int e = 0;
-  for (int P = 0; P < 81; P++)
-    for (int R = P; R < 81; R++) T.hmap[e++] = (uint16_t)((P << 7) | R);
+  for (int i = 0; i < NN; i++)
+    for (int j = i; j < NN; j++) T.pmap[e++] = (uint16_t)((i << 5) | j);
 }
 
 size_t assemble_sf_smem_bytes() { return sizeof(sf::Smem); }
@@ -489,7 +574,7 @@ static cudaError_t launch_sf_t(const AsmArgs &a, const SfTables *tb, const int *
   }
   const int grid = nelem < grid_cap ? nelem : grid_cap;
   if (grid <= 0) return cudaSuccess;
-  k<<<grid, 256, sm, st>>>(a, tb, elems, nelem);
+  k<<<grid, sf::NT, sm, st>>>(a, tb, elems, nelem);
   return cudaGetLastError();
 }
 

@@ -344,8 +344,8 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
   for (int c = 0; c < ncol; c++) {
     const int n = L.color_ptr[c + 1] - L.color_ptr[c];
     if (kp == 4)
-      e = launch_assemble_sf(a, L.energy != 0, d_sf, d_color_elems + L.color_ptr[c], n, tc_grid,
-                             st);
+      e = launch_assemble_sf(a, L.energy != 0, d_sf, d_color_elems + L.color_ptr[c], n,
+                             3 * num_sms, st);
     else if (kp == 3)
       e = launch_assemble_gemm(a, L.energy != 0, d_tab_iso, d_color_elems + L.color_ptr[c], n,
                                tc_grid, st);

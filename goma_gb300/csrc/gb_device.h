@@ -91,7 +91,7 @@ struct SfTables {
   double dref[27][27][3];
   int lex[27];
   int loc[27];
-  uint16_t hmap[81 * 82 / 2];
+  uint16_t pmap[27 * 28 / 2];  // node pairs i <= j, i << 5 | j
 };
 // species rows of 3-D elements by sum factorisation (gb_assemble_species.cu)
 cudaError_t launch_assemble_species_sf(const AsmArgs &a, bool energy, bool jac,
