@@ -129,65 +129,157 @@ __global__ void norms_final_kernel(int nblocks, const double *__restrict__ part,
   out[2] = mx;
 }
 
-// Partial dots of w with the k columns V[0..k) (column stride ld), kMdCols
-// columns per block row (blockIdx.y): a thread reads w once per group of
-// columns and keeps one running sum per column, and the block reduces all
-// of them with one barrier per halving.  Grid (nblocks, column groups);
-// block b's sum for column j goes to part[j * gridDim.x + b].
-static constexpr int kMdCols = 8;
-static constexpr int kMdBlocks = 2 * kRedBlocks;  // block rows of a column group
-template <class T>
-__global__ void __launch_bounds__(kRedThreads)
-    multidot_tile_kernel(int N, int k, const T *__restrict__ V, int64_t ld,
-                         const T *__restrict__ w, double *__restrict__ part) {
-  __shared__ double sh[kMdCols][kRedThreads];
-  using A = acc_t<T>;
-  const int j0 = blockIdx.y * kMdCols;
-  const int nc = min(kMdCols, k - j0);
-  A s[kMdCols];
-#pragma unroll
-  for (int c = 0; c < kMdCols; c++) s[c] = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const A wi = (A)w[i];
-#pragma unroll
-    for (int c = 0; c < kMdCols; c++)
-      if (c < nc) s[c] = fmx((A)V[(int64_t)(j0 + c) * ld + i], wi, s[c]);
+// Running sums of products.  FP64: one FMA chain.  FP32 data: the products
+// in FP32, summed with their rounding errors (Knuth's two-sum), so that a
+// thread may add many before it widens to FP64: the FP64 adds, at 1/64 of the
+// FP32 rate, were what bound the FP32 dots.
+struct SumF64 {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double a, double b) { s = fma(a, b, s); }
+  __device__ __forceinline__ double get() const { return s; }
+};
+struct SumF32 {
+  float s = 0.f, e = 0.f;
+  __device__ __forceinline__ void add(float a, float b) {
+    const float p = __fmul_rn(a, b), t = __fadd_rn(s, p), z = __fsub_rn(t, s);
+    e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z)));
+    s = t;
   }
+  __device__ __forceinline__ double get() const { return (double)s + (double)e; }
+};
+template <class T>
+struct SumOf {
+  using type = SumF64;
+};
+template <>
+struct SumOf<float> {
+  using type = SumF32;
+};
+
+// The warp's sums of v[0..4): 6 adds instead of 20, each step adding halves
+// of the lanes that keep different values.  Lane l returns the sum of
+// v[l >> 3].
+__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16, odd = lane & 8;
+  const double a = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+  const double b = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+  double c = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
 #pragma unroll
-  for (int c = 0; c < kMdCols; c++) sh[c][threadIdx.x] = (double)s[c];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+
+// Steps of the classical Gram-Schmidt passes against the k columns V[0..k)
+// (column stride ld):
+//   GS_DOTS      part = V^T w
+//   GS_SUB_DOTS  w -= V h, part = V^T w
+//   GS_SUB_NORM  w -= V h, part = w^T w
+// A block takes tiles of 128 rows and its eight warps share the columns, so
+// that a few thousand rows still fill the chip and a warp's sums need no
+// other warp; block b's sum for column j goes to part[j * gridDim.x + b].
+//
+// Bound by FP64 (N k FMA a step and half as many adds in the sums, at 2 a
+// clock and SM: 27 us for the dots at N = 160K, k = 67) and by loading V, 3
+// times where separate dots and updates load it 4 times.  The dots used to
+// keep one product a thread and add 256 of them in shared memory, more FP64
+// adds than products.  Both passes with the norm, N = 34K, k = 70 to 140:
+// dots 45 -> 9 us, update 14 -> 14 us with the second dots in it; N = 160K, k
+// = 67: dots 60 -> 34 us, update and dots 91 -> 55 us.
+enum { GS_DOTS, GS_SUB_DOTS, GS_SUB_NORM };
+static constexpr int kGsRows = 128;
+static constexpr int kGsBlocks = 8 * 152;  // two waves: 43 us with one at N = 160K
+template <class T, int OP>
+__global__ void __launch_bounds__(256, 4)
+    gs_kernel(int N, int k, const T *__restrict__ V, int64_t ld, const double *__restrict__ h,
+              T *__restrict__ w, double *__restrict__ part) {
+  using A = acc_t<T>;
+  constexpr int RPT = kGsRows / 32;
+  __shared__ A sub[8][kGsRows];
+  __shared__ A wn[kGsRows];
+  __shared__ double red[kGsRows / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const int ntile = (N + kGsRows - 1) / kGsRows;
+  double nrm = 0.0;
+  for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    const int i0 = tile * kGsRows + lane;
+    A wv[RPT];
+    if (OP != GS_DOTS) {
+      A s[RPT];
 #pragma unroll
-      for (int c = 0; c < kMdCols; c++) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
+      for (int r = 0; r < RPT; r++) s[r] = 0;
+#pragma unroll 4
+      for (int j = wp; j < k; j += 8) {
+        const A c = (A)h[j];
+        const T *v = V + j * ld + i0;
+#pragma unroll
+        for (int r = 0; r < RPT; r++)
+          if (i0 + 32 * r < N) s[r] = fmx(c, (A)v[32 * r], s[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < RPT; r++) sub[wp][lane + 32 * r] = s[r];
+      __syncthreads();
+      if (tid < kGsRows) {
+        const int i = tile * kGsRows + tid;
+        A t = 0;
+        if (i < N) {
+          t = (A)w[i];
+#pragma unroll
+          for (int q = 0; q < 8; q++) t -= sub[q][tid];
+          w[i] = (T)t;
+        }
+        wn[tid] = t;
+        if (OP == GS_SUB_NORM) nrm = sizeof(T) == 8 ? fma((double)t, (double)t, nrm)
+                                                    : nrm + (double)(t * t);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < RPT; r++) wv[r] = wn[lane + 32 * r];
+    } else {
+#pragma unroll
+      for (int r = 0; r < RPT; r++) wv[r] = i0 + 32 * r < N ? (A)w[i0 + 32 * r] : (A)0;
+    }
+    for (int j0 = 4 * wp; OP != GS_SUB_NORM && j0 < k; j0 += 32) {
+      double v[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const T *x = V + (int64_t)(j0 + c) * ld + i0;
+        typename SumOf<T>::type s;
+#pragma unroll
+        for (int r = 0; r < RPT; r++)
+          if (j0 + c < k && i0 + 32 * r < N) s.add((A)x[32 * r], wv[r]);
+        v[c] = s.get();
+      }
+      const double sum = warp_sum4(v);
+      const int j = j0 + (lane >> 3);
+      if ((lane & 7) == 0 && j < k) {
+        double *p = part + (int64_t)j * gridDim.x + blockIdx.x;
+        *p = tile == blockIdx.x ? sum : *p + sum;
+      }
+    }
+  }
+  if (OP == GS_SUB_NORM) {
+    if (wp < kGsRows / 32) {
+      nrm = warp_sum(nrm);
+      if (lane == 0) red[wp] = nrm;
     }
     __syncthreads();
+    if (tid == 0) part[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
   }
-  if (threadIdx.x < nc) part[(int64_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = sh[threadIdx.x][0];
 }
 
-// out[j] = sum over the nblocks partial sums of column j, a warp per column
-__global__ void multidot_final_kernel(int k, int nblocks, const double *__restrict__ part,
-                                      double *__restrict__ out) {
-  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (j >= k) return;
+// out[j] = sum over the nblocks partial sums of column j, a block per column
+__global__ void __launch_bounds__(128)
+    multidot_final_kernel(int nblocks, const double *__restrict__ part, double *__restrict__ out) {
+  __shared__ double red[4];
+  const int j = blockIdx.x;
   double s = 0.0;
-  for (int b = lane; b < nblocks; b += 32) s += part[(int64_t)j * nblocks + b];
-  s = warp_sum(s);
-  if (lane == 0) out[j] = s;
-}
-
-// w -= sum_j h[j] V[:, j]
-template <class T>
-__global__ void gemv_sub_kernel(int N, int k, const T *__restrict__ V, int64_t ld,
-                                const double *__restrict__ h, T *__restrict__ w) {
-  using A = acc_t<T>;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    A s = (A)w[i];
 #pragma unroll 4
-    for (int j = 0; j < k; j++) s = fmx((A)-h[j], (A)V[j * ld + i], s);
-    w[i] = (T)s;
-  }
+  for (int b = threadIdx.x; b < nblocks; b += 128) s += part[(int64_t)j * nblocks + b];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) out[j] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // y = sum_j c[j] V[:, j]  (c on device)
@@ -203,12 +295,43 @@ __global__ void gemv_kernel(int N, int k, const T *__restrict__ V, int64_t ld,
   }
 }
 
-template <class T>
-__global__ void scale_copy_kernel(int N, const T *x, const double *__restrict__ alpha_inv, T *y) {
+// y = x / norm (0 where the norm is 0), and the same to y2, the operand of the
+// preconditioner.  The norm: norm[0], or with nparts > 0 the root of the sum
+// of part[0..nparts), formed alike by every block and kept in norm[0].
+template <class T, class T2>
+__global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *__restrict__ part,
+                                  double *norm, T *y, T2 *__restrict__ y2) {
   using A = acc_t<T>;
-  const A a = (A)(alpha_inv[0] != 0.0 ? 1.0 / alpha_inv[0] : 0.0);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-    y[i] = (T)((A)x[i] * a);
+  __shared__ double red[kRedThreads / 32];
+  __shared__ double inv;
+  if (nparts > 0) {
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nparts; b += kRedThreads) s += part[b];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+  }
+  // one thread: the root and the quotient by all of them kept the FP64 pipe
+  // longer than the copy takes
+  if (threadIdx.x == 0) {
+    double nv;
+    if (nparts > 0) {
+      nv = 0.0;
+      for (int q = 0; q < kRedThreads / 32; q++) nv += red[q];
+      nv = sqrt(nv);
+      if (blockIdx.x == 0) norm[0] = nv;
+    } else {
+      nv = norm[0];
+    }
+    inv = nv != 0.0 ? 1.0 / nv : 0.0;
+  }
+  __syncthreads();
+  const A a = (A)inv;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    const T v = (T)((A)x[i] * a);
+    y[i] = v;
+    if (y2) y2[i] = (T2)v;
+  }
 }
 
 __global__ void axpy_kernel(int N, double a, const double *__restrict__ x, double *__restrict__ y) {
@@ -703,7 +826,7 @@ int Solver::init(Context *c, int krylov) {
   }
   GB_CU(cudaMalloc(&d_lu, sizeof(double) * nnz), "ILU factors");
   GB_CU(cudaMalloc(&d_scale, sizeof(double) * N), "scale");
-  const size_t wk = (size_t)(kRedBlocks * 3 + (krylov + 2) * kMdBlocks + 4 * (krylov + 2) + 96);
+  const size_t wk = (size_t)(kRedBlocks * 3 + (krylov + 2) * kGsBlocks + 4 * (krylov + 2) + 96);
   GB_CU(cudaMalloc(&d_work, sizeof(double) * wk), "work");
   GB_CU(cudaMallocHost(&h_work, sizeof(double) * 4 * (krylov + 2) + 64 * sizeof(double)), "host");
   GB_CU(cudaMalloc(&d_V, sizeof(double) * (size_t)(krylov + 1) * N), "Krylov basis");
@@ -1010,9 +1133,10 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
   const int64_t ld = N;
   double *dred = S.d_work;                           // partials
   double *dh = S.d_work + kRedBlocks * 3 + 16;       // (m+2) results
-  double *dpart = dh + (m + 2) * 2 + 8;              // (m+2) * kMdBlocks
-  // the row-parallel kernels (w -= V h, y = V c) get a thread per unknown:
-  // enough loads in flight to stream the basis at HBM speed
+  double *dpart = dh + (m + 2) * 2 + 8;              // (m+2) * kGsBlocks
+  const int gs_blocks = std::min((N + kGsRows - 1) / kGsRows, kGsBlocks);
+  // y = V c gets a thread per unknown: enough loads in flight to stream the
+  // basis at HBM speed
   const int rows_grid = (N + kRedThreads - 1) / kRedThreads;
   double *hh = S.h_work;
   std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), g(m + 1), y(m);
@@ -1023,6 +1147,14 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     GB_CU(cudaStreamSynchronize(st), "norm sync");
     *out = hh[0];
     return 0;
+  };
+  // v = src / norm, and the preconditioner's copy of it
+  auto basis_vector = [&](const T *src, int nparts, const double *part, double *nrm, T *v) {
+    if (flexible)
+      scale_copy_kernel<T, float><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm,
+                                                                      v, S.d_t32);
+    else
+      scale_copy_kernel<T, T><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm, v, t);
   };
   GB_CU(cudaMemsetAsync(x, 0, sizeof(T) * N, st), "x0");
   double bnorm;
@@ -1038,7 +1170,7 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     // V0 = r / beta (dh[0] = beta)
     hh[0] = beta;
     GB_CU(cudaMemcpyAsync(dh, hh, sizeof(double), cudaMemcpyHostToDevice, st), "beta");
-    scale_copy_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(N, V, dh, V);
+    basis_vector(V, 0, nullptr, dh, V);
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int j = 0;
@@ -1047,34 +1179,25 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
       const T *zj = t;  // M^-1 v_j
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
-          // the preconditioner in FP32: v_j -> FP32, sweeps, z_j kept in FP64
-          to_f32_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, V + j * ld, S.d_t32);
+          // the preconditioner in FP32, z_j kept in FP64
           if (S.apply_prec32(st)) return -1;
           to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + j * ld);
           zj = S.d_Z + j * ld;
         }
       }
       if (!flexible) {
-        GB_CU(cudaMemcpyAsync(t, V + j * ld, sizeof(T) * N, cudaMemcpyDeviceToDevice, st), "t");
         if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
       }
       GB_CU(spmv<T>(C, lpr, A, zj, w, st), "spmv");
       // CGS2 on the device; the host reads both passes and the norm in one copy
       std::vector<double> hcol(j + 2, 0.0);
       double *dh1 = dh, *dh2 = dh + (m + 2), *dnrm = dh + 2 * (m + 2);
-      multidot_tile_kernel<T><<<dim3(kMdBlocks, (j + kMdCols) / kMdCols), kRedThreads, 0, st>>>(
-          N, j + 1, V, ld, w, dpart);
-      // a warp per coefficient, eight a block
-      const int fin = (j + 1 + 7) / 8;
-      multidot_final_kernel<<<fin, 256, 0, st>>>(j + 1, kMdBlocks, dpart, dh1);
-      gemv_sub_kernel<T><<<rows_grid, kRedThreads, 0, st>>>(N, j + 1, V, ld, dh1, w);
-      multidot_tile_kernel<T><<<dim3(kMdBlocks, (j + kMdCols) / kMdCols), kRedThreads, 0, st>>>(
-          N, j + 1, V, ld, w, dpart);
-      multidot_final_kernel<<<fin, 256, 0, st>>>(j + 1, kMdBlocks, dpart, dh2);
-      gemv_sub_kernel<T><<<rows_grid, kRedThreads, 0, st>>>(N, j + 1, V, ld, dh2, w);
-      norms_partial_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(N, w, dred);
-      norms_final_kernel<<<1, 32, 0, st>>>(kRedBlocks, dred, dnrm);
-      scale_copy_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(N, w, dnrm, V + (j + 1) * ld);
+      gs_kernel<T, GS_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, nullptr, w, dpart);
+      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh1);
+      gs_kernel<T, GS_SUB_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh1, w, dpart);
+      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh2);
+      gs_kernel<T, GS_SUB_NORM><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh2, w, dpart);
+      basis_vector(w, gs_blocks, dpart, dnrm, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "Arnoldi step");
       GB_CU(cudaMemcpyAsync(hh, dh, sizeof(double) * (2 * (m + 2) + 1), cudaMemcpyDeviceToHost,
                             st), "h");
@@ -1141,47 +1264,92 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
 // convergence test; SpMV and the (block-diagonal) ILU(0) serve all blocks
 // at once.
 
-// part[t][j] = sum over tile t of V_j . w, j < k (k <= 32)
-template <class T>
-__global__ void seg_dots_kernel(int k, const T *__restrict__ V, int64_t ld,
-                                const T *__restrict__ w, const int64_t *__restrict__ tbeg,
-                                const int64_t *__restrict__ tend, double *__restrict__ part) {
-  __shared__ double red[8];
-  const int t = blockIdx.x, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int64_t b = tbeg[t], e = tend[t];
+// The Gram-Schmidt steps of gs_kernel on tiles of blocks: part[t][j] = the
+// sum over tile t of V_j . w (GS_SUB_NORM: w . w in part[t][0]), j < k <= 32,
+// coefficients c[s][j] of the tile's block s.  A thread keeps its 8 rows of w
+// in registers over all columns, and a warp adds four columns at once.  One
+// column at a time the dots waited for two barriers each (37 us for 32
+// blocks of 2-D meshes, k = 16; now 21 us, 23 us with the update, which took
+// 20 us by itself).
+static constexpr int kSegRows = 8;  // a tile has at most 8 x 256 unknowns
+template <class T, int OP>
+__global__ void __launch_bounds__(256, 2)
+    seg_gs_kernel(int k, const T *__restrict__ V, int64_t ld, const double *__restrict__ c,
+                  T *__restrict__ w, const int *__restrict__ tseg,
+                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
+                  double *__restrict__ part) {
   using A = acc_t<T>;
-  for (int j = 0; j < k; j++) {
-    A acc = 0;
-    for (int64_t i = b + threadIdx.x; i < e; i += blockDim.x)
-      acc = fmx((A)V[j * ld + i], (A)w[i], acc);
-    const double sum = warp_sum((double)acc);
-    if (lane == 0) red[wp] = sum;
+  __shared__ double red[8][32];
+  __shared__ double cs[32];
+  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const int64_t b = tbeg[t] + tid, e = tend[t];
+  A wv[kSegRows];
+#pragma unroll
+  for (int r = 0; r < kSegRows; r++) wv[r] = b + 256 * r < e ? (A)w[b + 256 * r] : (A)0;
+  if (OP != GS_DOTS) {
+    if (tid < 32) cs[tid] = tid < k ? c[tseg[t] * 32 + tid] : 0.0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0.0;
-      for (int q = 0; q < (int)(blockDim.x >> 5); q++) tot += red[q];
-      part[(int64_t)t * 32 + j] = tot;
+    A s[kSegRows];
+#pragma unroll
+    for (int r = 0; r < kSegRows; r++) s[r] = 0;
+#pragma unroll 2
+    for (int j = 0; j < k; j++) {
+      const T *v = V + j * ld + b;
+      const A cj = (A)cs[j];
+#pragma unroll
+      for (int r = 0; r < kSegRows; r++)
+        if (b + 256 * r < e) s[r] = fmx(cj, (A)v[256 * r], s[r]);
     }
-    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSegRows; r++) {
+      wv[r] -= s[r];
+      if (b + 256 * r < e) w[b + 256 * r] = (T)wv[r];
+    }
+  }
+  const int nd = OP == GS_SUB_NORM ? 1 : k;
+  for (int j0 = 0; j0 < nd; j0 += 4) {
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      typename SumOf<T>::type s;
+      if (OP == GS_SUB_NORM) {
+        if (q == 0)
+#pragma unroll
+          for (int r = 0; r < kSegRows; r++) s.add(wv[r], wv[r]);
+      } else {
+        const T *x = V + (int64_t)(j0 + q) * ld + b;
+#pragma unroll
+        for (int r = 0; r < kSegRows; r++)
+          if (j0 + q < k && b + 256 * r < e) s.add((A)x[256 * r], wv[r]);
+      }
+      v[q] = s.get();
+    }
+    const double sum = warp_sum4(v);
+    if ((lane & 7) == 0) red[wp][j0 + (lane >> 3)] = sum;
+  }
+  __syncthreads();
+  if (tid < nd) {
+    double sum = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) sum += red[q][tid];
+    part[(int64_t)t * 32 + tid] = sum;
   }
 }
 
-// out[s][j] = sum over the tiles of block s of part[t][j]; one warp per block
+// out[s][j] = sum over the tiles of block s of part[t][j]; a warp per (s, j)
 __global__ void seg_reduce_kernel(int nseg, int k, const int *__restrict__ tptr,
                                   const double *__restrict__ part, double *__restrict__ out) {
-  const int sg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (sg >= nseg) return;
-  for (int j = 0; j < k; j++) {
-    double sum = 0.0;
-    for (int t = tptr[sg] + lane; t < tptr[sg + 1]; t += 32) sum += part[(int64_t)t * 32 + j];
-    sum = warp_sum(sum);
-    if (lane == 0) out[sg * 32 + j] = sum;
-  }
+  const int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (u >= nseg * k) return;
+  const int sg = u / k, j = u - sg * k;
+  double sum = 0.0;
+  for (int t = tptr[sg] + lane; t < tptr[sg + 1]; t += 32) sum += part[(int64_t)t * 32 + j];
+  sum = warp_sum(sum);
+  if (lane == 0) out[sg * 32 + j] = sum;
 }
 
-// w -= sum_j c[s][j] V_j on block s (c = the reduced dots), or with
-// ACCUMULATE = false: y = sum_j c[s][j] V_j
-template <class T, bool SUB>
+// y = sum_j c[s][j] V_j on block s
+template <class T>
 __global__ void seg_gemv_kernel(int k, const T *__restrict__ V, int64_t ld,
                                 const double *__restrict__ c, const int *__restrict__ tseg,
                                 const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
@@ -1195,22 +1363,31 @@ __global__ void seg_gemv_kernel(int k, const T *__restrict__ V, int64_t ld,
   for (int64_t i = tbeg[t] + threadIdx.x; i < tend[t]; i += blockDim.x) {
     A acc = 0;
     for (int j = 0; j < k; j++) acc = fmx((A)cs[j], (A)V[j * ld + i], acc);
-    y[i] = SUB ? (T)((A)y[i] - acc) : (T)acc;
+    y[i] = (T)acc;
   }
 }
 
 // dst = src * alpha[s] on block s; alpha = 1 / sqrt(norm2[s]) for active
-// blocks with a nonzero norm, else 0 (from the reduced norms when scale is NULL)
-template <class T>
-__global__ void seg_scale_kernel(const T *__restrict__ src, const double *__restrict__ norm2,
+// blocks with a nonzero norm, else 0; the same to dst2, the operand of the
+// preconditioner
+template <class T, class T2>
+__global__ void seg_scale_kernel(const T *src, const double *__restrict__ norm2,
                                  const int *__restrict__ active, const int *__restrict__ tseg,
                                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
-                                 T *__restrict__ dst) {
+                                 T *dst, T2 *__restrict__ dst2) {
   const int t = blockIdx.x, sg = tseg[t];
-  const double n2 = norm2[sg * 32];
-  const acc_t<T> a = (acc_t<T>)((active[sg] && n2 > 0.0) ? 1.0 / sqrt(n2) : 0.0);
-  for (int64_t i = tbeg[t] + threadIdx.x; i < tend[t]; i += blockDim.x)
-    dst[i] = (T)((acc_t<T>)src[i] * a);
+  __shared__ double inv;
+  if (threadIdx.x == 0) {
+    const double n2 = norm2[sg * 32];
+    inv = (active[sg] && n2 > 0.0) ? 1.0 / sqrt(n2) : 0.0;
+  }
+  __syncthreads();
+  const acc_t<T> a = (acc_t<T>)inv;
+  for (int64_t i = tbeg[t] + threadIdx.x; i < tend[t]; i += blockDim.x) {
+    const T v = (T)((acc_t<T>)src[i] * a);
+    dst[i] = v;
+    dst2[i] = (T2)v;
+  }
 }
 
 template <class T>
@@ -1229,11 +1406,23 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
   const int64_t ld = N;
   double *o1 = S.d_segout, *o2 = o1 + 32 * ns, *o3 = o2 + 32 * ns;
   double *h1 = S.h_segout, *h2 = h1 + 32 * ns, *h3 = h2 + 32 * ns;
-  const int rblocks = (ns + 7) / 8;
-  auto dots = [&](int k, const T *Vb, const T *wv, double *out) {
-    seg_dots_kernel<T><<<nt, 256, 0, st>>>(k, Vb, ld, wv, S.d_tile_beg, S.d_tile_end,
-                                           S.d_segpart);
-    seg_reduce_kernel<<<rblocks, 256, 0, st>>>(ns, k, S.d_tile_ptr, S.d_segpart, out);
+  auto reduce = [&](int k, double *out) {
+    seg_reduce_kernel<<<(ns * k + 7) / 8, 256, 0, st>>>(ns, k, S.d_tile_ptr, S.d_segpart, out);
+  };
+  // w . v on every block
+  auto dot1 = [&](const T *v, T *wv, double *out) {
+    seg_gs_kernel<T, GS_DOTS><<<nt, 256, 0, st>>>(1, v, ld, nullptr, wv, S.d_tile_seg,
+                                                  S.d_tile_beg, S.d_tile_end, S.d_segpart);
+    reduce(1, out);
+  };
+  // v = src / norm per block, and the preconditioner's copy of it
+  auto basis_vector = [&](const T *src, T *v) {
+    if (flexible)
+      seg_scale_kernel<T, float><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
+                                                     S.d_tile_beg, S.d_tile_end, v, S.d_t32);
+    else
+      seg_scale_kernel<T, T><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
+                                                 S.d_tile_beg, S.d_tile_end, v, t);
   };
   std::vector<int> active(ns, 1), done(ns, 0);
   std::vector<double> bnorm(ns), beta(ns), coef(32 * (size_t)ns);
@@ -1246,7 +1435,8 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
     return 0;
   };
   GB_CU(cudaMemsetAsync(x, 0, sizeof(T) * N, st), "x0");
-  dots(1, b, b, o3);
+  GB_CU(cudaMemcpyAsync(V, b, sizeof(T) * N, cudaMemcpyDeviceToDevice, st), "r0");
+  dot1(V, V, o3);
   GB_CU(cudaMemcpyAsync(h3, o3, sizeof(double) * 32 * ns, cudaMemcpyDeviceToHost, st), "norms");
   GB_CU(cudaStreamSynchronize(st), "norms");
   bool any = false;
@@ -1259,13 +1449,11 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
   *its = 0;
   *relres = 0.0;
   if (!any) return 0;
-  GB_CU(cudaMemcpyAsync(V, b, sizeof(T) * N, cudaMemcpyDeviceToDevice, st), "r0");
   int total = 0;
   while (true) {
     if (upload_active()) return -1;
     // V0 = r / beta per block (o3 holds the squared norms of r)
-    seg_scale_kernel<T><<<nt, 256, 0, st>>>(V, o3, S.d_segactive, S.d_tile_seg, S.d_tile_beg,
-                                            S.d_tile_end, V);
+    basis_vector(V, V);
     for (int sg = 0; sg < ns; sg++) {
       std::fill(&g[(size_t)sg * (m + 1)], &g[(size_t)sg * (m + 1)] + m + 1, 0.0);
       g[(size_t)sg * (m + 1)] = beta[sg];
@@ -1278,26 +1466,25 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
           // the (block-diagonal) preconditioner in FP32, z_j kept in FP64
-          to_f32_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, V + j * ld, S.d_t32);
           if (S.apply_prec32(st)) return -1;
           to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + j * ld);
           zj = S.d_Z + j * ld;
         }
       }
       if (!flexible) {
-        GB_CU(cudaMemcpyAsync(t, V + j * ld, sizeof(T) * N, cudaMemcpyDeviceToDevice, st), "t");
         if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
       }
       GB_CU(spmv<T>(C, lpr, A, zj, w, st), "spmv");
-      dots(j + 1, V, w, o1);
-      seg_gemv_kernel<T, true><<<nt, 256, 0, st>>>(j + 1, V, ld, o1, S.d_tile_seg,
-                                                   S.d_tile_beg, S.d_tile_end, w);
-      dots(j + 1, V, w, o2);
-      seg_gemv_kernel<T, true><<<nt, 256, 0, st>>>(j + 1, V, ld, o2, S.d_tile_seg,
-                                                   S.d_tile_beg, S.d_tile_end, w);
-      dots(1, w, w, o3);
-      seg_scale_kernel<T><<<nt, 256, 0, st>>>(w, o3, S.d_segactive, S.d_tile_seg, S.d_tile_beg,
-                                              S.d_tile_end, V + (j + 1) * ld);
+      seg_gs_kernel<T, GS_DOTS><<<nt, 256, 0, st>>>(j + 1, V, ld, nullptr, w, S.d_tile_seg,
+                                                    S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      reduce(j + 1, o1);
+      seg_gs_kernel<T, GS_SUB_DOTS><<<nt, 256, 0, st>>>(j + 1, V, ld, o1, w, S.d_tile_seg,
+                                                        S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      reduce(j + 1, o2);
+      seg_gs_kernel<T, GS_SUB_NORM><<<nt, 256, 0, st>>>(j + 1, V, ld, o2, w, S.d_tile_seg,
+                                                        S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      reduce(1, o3);
+      basis_vector(w, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "batched Arnoldi step");
       GB_CU(cudaMemcpyAsync(h1, o1, sizeof(double) * 3 * 32 * ns, cudaMemcpyDeviceToHost, st),
             "h");
@@ -1360,12 +1547,12 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
       if constexpr (std::is_same<T, double>::value) {
         // flexible: x += Z y, the preconditioned vectors as they were applied
         if (flexible)
-          seg_gemv_kernel<T, false><<<nt, 256, 0, st>>>(kmax, S.d_Z, ld, S.d_segcoef,
+          seg_gemv_kernel<T><<<nt, 256, 0, st>>>(kmax, S.d_Z, ld, S.d_segcoef,
                                                         S.d_tile_seg, S.d_tile_beg,
                                                         S.d_tile_end, t);
       }
       if (!flexible) {
-        seg_gemv_kernel<T, false><<<nt, 256, 0, st>>>(kmax, V, ld, S.d_segcoef, S.d_tile_seg,
+        seg_gemv_kernel<T><<<nt, 256, 0, st>>>(kmax, V, ld, S.d_segcoef, S.d_tile_seg,
                                                       S.d_tile_beg, S.d_tile_end, t);
         if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
       }
@@ -1374,7 +1561,7 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
     // true residual per block
     GB_CU(spmv<T>(C, lpr, A, x, V, st), "spmv");
     sub_from_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(N, b, V);
-    dots(1, V, V, o3);
+    dot1(V, V, o3);
     GB_CU(cudaMemcpyAsync(h3, o3, sizeof(double) * 32 * ns, cudaMemcpyDeviceToHost, st), "norms");
     GB_CU(cudaStreamSynchronize(st), "norms");
     double worst = 0.0;
