@@ -10,9 +10,8 @@
 // live in one flat FP32 buffer (and gradients / Adam moments in three more),
 // so the host can read, write and checksum them in one copy.
 //
-// GEMMs are tiled SIMT FP32 (64 x 64 tiles, 4 x 4 per thread): at width 256
-// and batches of a few thousand points one training step is a few GFLOP, far
-// below the time of one Newton solve.
+// The products run on the FP32 pipe in FP32 FMA, a sum over k in ascending
+// order: the predictor's accuracy is that of FP32 arithmetic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,173 +27,394 @@
 
 namespace gb {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int TM = 64, TN = 64, TK = 32;
 constexpr int kMaxSplit = 32;  // batch splits of the weight-gradient product
+constexpr int kNarrow = 8;     // widths up to this take the narrow kernels
 
-// C[M][N] = A[M][K] * B^T where B is [N][K]  (i.e. X W^T), + bias[N],
-// optional tanh.  Row-major everything.
-__global__ void __launch_bounds__(256)
-    gemm_xwT_kernel(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B,
-                    const float *__restrict__ bias, float *__restrict__ C, int act) {
-  __shared__ float As[TK][TM + 4];
-  __shared__ float Bs[TK][TN + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    for (int t = threadIdx.x; t < TM * TK; t += 256) {
-      const int mm = t / TK, kk = t % TK;
-      const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? A[(int64_t)gm * K + gk] : 0.f;
-      const int gn = n0 + mm;
-      Bs[kk][mm] = (gn < N && gk < K) ? B[(int64_t)gn * K + gk] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; kk++) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+// ---- tiled product C[M][N] = sum_k A(m, k) B(k, n)
+//
+// Operand tiles (64 rows, 32 k) go through registers to shared memory as
+// S[k][row], rows in 16-byte pieces moved by 4 * (k / 4 % 8): the transposing
+// stores of k-contiguous operands and all loads then hit distinct banks.  256
+// threads in two groups, each with half of a tile's k and 8 x 4 outputs a
+// thread, in packed FMA (fma.rn.f32x2, 15 % faster than single ones): 16 FMA
+// instructions per 3 shared loads.  At the end the groups add their sums and
+// each keeps half of the rows.  The next tile's global loads are in flight
+// while a tile is multiplied.
+//
+// Bound by the FP32 pipe, 128 FMA a clock and SM: 4096 x 256 x 256 takes 7.2
+// us at that rate.  64 x 64 tiles make 256 blocks of it, at most two on an SM
+// (84 %), and the second group keeps the pipe fed with so few blocks: 14.5
+// us, 16.5 us with one group, 21.5 us (forward 25 us) with 4 x 4 outputs, twice
+// the shared loads and no prefetch.  8 x 8 outputs in four groups: 17.5 us.
+// 34,306 rows: 100 us, 58 % of the pipe.
+
+// A thread's two pieces of 16 bytes of the tiles of one operand.  KC:
+// P[row][k], ld = row stride; else P[k][row], ld = k stride.  Whole aligned
+// tiles take the short path: the checks of the others were 40 % of the
+// instructions.
+template <bool KC>
+struct TileLoad {
+  const float *p;  // the first piece
+  int64_t second;  // the other from it
+  int64_t ld;
+  int r, k, rows, kend;
+  bool whole;
+  __device__ __forceinline__ TileLoad(const float *P, int ld_, int r0, int rows_, int k0, int kend_,
+                                      bool vec)
+      : ld(ld_), rows(rows_), kend(kend_), whole(vec && r0 + TM <= rows_) {
+    const int t = threadIdx.x;
+    r = KC ? r0 + t / (TK / 4) : r0 + (t % 16) * 4;
+    k = KC ? k0 + (t % (TK / 4)) * 4 : k0 + t / 16;
+    p = KC ? P + (int64_t)r * ld + k : P + (int64_t)k * ld + r;
+    second = KC ? 32 * ld : TK / 2 * ld;
   }
+  // the tile at k0, then on to the next
+  __device__ __forceinline__ void next(int k0, float4 (&v)[2]) {
+    if (whole && k0 + TK <= kend) {
+      v[0] = *reinterpret_cast<const float4 *>(p);
+      v[1] = *reinterpret_cast<const float4 *>(p + second);
+    } else {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
+      for (int u = 0; u < 2; u++) {
+        const float *x = p + u * second;
+        const int left = KC ? (r + 32 * u < rows ? kend - k : 0)
+                            : (k + TK / 2 * u < kend ? rows - r : 0);
+        v[u].x = left > 0 ? x[0] : 0.f;
+        v[u].y = left > 1 ? x[1] : 0.f;
+        v[u].z = left > 2 ? x[2] : 0.f;
+        v[u].w = left > 3 ? x[3] : 0.f;
+      }
+    }
+    k += TK;
+    p += KC ? TK : TK * ld;
+  }
+};
+
+// the move of the pieces of row k
+__device__ __forceinline__ int tile_swz(int k) { return ((k >> 2) & 7) * 4; }
+
+template <bool KC>
+__device__ __forceinline__ void tile_store(float (*S)[TM], const float4 (&v)[2]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    if (KC) {
+      const int k = (t % 8) * 4, r = (t / 8 + 32 * u) ^ tile_swz(k);
+      S[k][r] = v[u].x;
+      S[k + 1][r] = v[u].y;
+      S[k + 2][r] = v[u].z;
+      S[k + 3][r] = v[u].w;
+    } else {
+      const int k = t / 16 + 16 * u, r = ((t % 16) * 4) ^ tile_swz(k);
+      *reinterpret_cast<float4 *>(&S[k][r]) = v[u];
+    }
+  }
+}
+
+// two FP32 FMA, each rounded like fmaf, and two adds
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a,
+                                     unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long dup2(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 split2(unsigned long long x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+
+// MLP_FORWARD  C = A W^T + E[n], with act: tanh of it   (A [M][K], W [N][K])
+// MLP_BACK     C = (A W) (1 - E[m][n]^2)                (A [M][K], W [K][N])
+// MLP_GRAD     split z of the sum over the batch k in chunks of kchunk, A
+//              [K][M] and B [K][N], to C + z (M N + M), followed by the split's
+//              sums of A over k (the bias gradient); grad_sum_kernel adds the
+//              splits in a fixed order, so the result is deterministic
+enum { MLP_FORWARD, MLP_BACK, MLP_GRAD };
+
+template <int OP>
+__global__ void __launch_bounds__(256, 2)
+    mlp_gemm_kernel(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B,
+                    const float *__restrict__ E, float *__restrict__ C, int act, int kchunk,
+                    bool vec_a, bool vec_b, bool vec_c) {
+  constexpr bool AK = OP != MLP_GRAD, BK = OP == MLP_FORWARD;
+  union Smem {
+    float t[2][2][TK][TM];         // buffer, operand
+    unsigned long long x[8][256];  // the groups' exchange
+    float s[256];
+  };
+  __shared__ __align__(16) Smem S;
+  const int tid = threadIdx.x, lane = tid & 31, wp = (tid >> 5) & 3, g = tid >> 7;
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  const int mi = (wp >> 1) * 32 + (lane >> 3) * 8, ni = (wp & 1) * 32 + (lane & 7) * 4;
+  const int kb = OP == MLP_GRAD ? blockIdx.z * kchunk : 0;
+  const int ke = OP == MLP_GRAD ? min(K, kb + kchunk) : K;
+  const int lda = AK ? K : M, ldb = BK ? K : N;
+  if (OP == MLP_GRAD) C += (int64_t)blockIdx.z * ((int64_t)M * N + M);
+  unsigned long long acc[4][4] = {};  // row pair i, column j
+  float cs = 0.f;
+  float4 va[2], vb[2];
+  TileLoad<AK> la(A, lda, m0, M, kb, ke, vec_a);
+  TileLoad<BK> lb(B, ldb, n0, N, kb, ke, vec_b);
+  la.next(kb, va);
+  lb.next(kb, vb);
+  int buf = 0;
+  for (int k0 = kb; k0 < ke; k0 += TK, buf ^= 1) {
+    float(*As)[TM] = S.t[buf][0], (*Bs)[TN] = S.t[buf][1];
+    tile_store<AK>(As, va);
+    tile_store<BK>(Bs, vb);
+    __syncthreads();
+    if (k0 + TK < ke) {
+      la.next(k0 + TK, va);
+      lb.next(k0 + TK, vb);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {  // four k with the same moves
+      const int k4 = g * 16 + q * 4, sw = tile_swz(k4);
+      const float *pa0 = &As[k4][mi ^ sw], *pa1 = &As[k4][(mi + 4) ^ sw];
+      const float *pb = &Bs[k4][ni ^ sw];
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++) {
+        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(pa0 + kk * TM);
+        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(pa1 + kk * TM);
+        const float4 b = *reinterpret_cast<const float4 *>(pb + kk * TN);
+        const unsigned long long a[4] = {a0.x, a0.y, a1.x, a1.y};
+        const unsigned long long d[4] = {dup2(b.x), dup2(b.y), dup2(b.z), dup2(b.w)};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) fma2(acc[i][j], a[i], d[j]);
+      }
+    }
+    if (OP == MLP_GRAD && blockIdx.x == 0) {  // sums of A: a column, eight k
+      const int k8 = (tid >> 6) * 8;
+      float ts = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; k++) ts += As[k8 + k][(tid & 63) ^ tile_swz(k8 + k)];
+      cs += ts;
+    }
+    // the buffer after next is written only after the next barrier
+  }
+  // group 0 keeps the first four rows of the groups' sums, group 1 the others
+  unsigned long long r[2][4];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) S.x[i * 4 + j][tid] = g ? acc[i][j] : acc[i + 2][j];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      r[i][j] = add2(g ? acc[i + 2][j] : acc[i][j], S.x[i * 4 + j][tid ^ 128]);
+  const int gm0 = m0 + mi + 4 * g, gn = n0 + ni;
+  float v[4][4];
+#pragma unroll
+  for (int i = 0; i < 2; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn >= N) continue;
-      float v = acc[i][j] + (bias ? bias[gn] : 0.f);
+      const float2 x = split2(r[i][j]);
+      v[2 * i][j] = x.x;
+      v[2 * i + 1][j] = x.y;
+    }
+  if (OP == MLP_FORWARD) {
+    float e[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) e[j] = gn + j < N ? E[gn + j] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        v[i][j] += e[j];
+        if (act) v[i][j] = tanhf(v[i][j]);
+      }
+  }
+  // whole tiles in pieces of 16 bytes
+  if (vec_c && m0 + TM <= M && n0 + TN <= N) {
+    if (OP == MLP_BACK) {
+      float4 h[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        h[i] = *reinterpret_cast<const float4 *>(E + (int64_t)(gm0 + i) * N + gn);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        v[i][0] *= 1.f - h[i].x * h[i].x;
+        v[i][1] *= 1.f - h[i].y * h[i].y;
+        v[i][2] *= 1.f - h[i].z * h[i].z;
+        v[i][3] *= 1.f - h[i].w * h[i].w;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *reinterpret_cast<float4 *>(C + (int64_t)(gm0 + i) * N + gn) =
+          make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+  } else {
+    for (int i = 0; i < 4; i++)
+      for (int j = 0; j < 4; j++) {
+        if (gm0 + i >= M || gn + j >= N) continue;
+        const int64_t o = (int64_t)(gm0 + i) * N + gn + j;
+        C[o] = OP == MLP_BACK ? v[i][j] * (1.f - E[o] * E[o]) : v[i][j];
+      }
+  }
+  if (OP == MLP_GRAD && blockIdx.x == 0) {
+    __syncthreads();
+    S.s[tid] = cs;
+    __syncthreads();
+    if (tid < TM && m0 + tid < M)
+      C[(int64_t)M * N + m0 + tid] =
+          (S.s[tid] + S.s[64 + tid]) + (S.s[128 + tid] + S.s[192 + tid]);
+  }
+}
+
+// ---- layers with at most kNarrow outputs or inputs, where a 64 x 64 tile
+// would be nearly empty
+
+// C[M][N] = A[M][K] W[N][K]^T + bias (tanh): a warp per row, lanes over k
+// (4096 x 1 x 256: 4 us, 10 us as a tile)
+__global__ void __launch_bounds__(256)
+    mlp_forward_narrow_kernel(int M, int N, int K, const float *__restrict__ A,
+                              const float *__restrict__ W, const float *__restrict__ bias,
+                              float *__restrict__ C, int act) {
+  const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (m >= M) return;
+  float s[kNarrow] = {};
+  const float *a = A + (int64_t)m * K;
+  for (int k = lane; k < K; k += 32) {
+    const float x = a[k];
+#pragma unroll
+    for (int j = 0; j < kNarrow; j++)
+      if (j < N) s[j] = fmaf(x, __ldg(W + (int64_t)j * K + k), s[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < kNarrow; j++)
+    if (j < N) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+      float v = s[j] + bias[j];
       if (act) v = tanhf(v);
-      C[(int64_t)gm * N + gn] = v;
+      if (lane == 0) C[(int64_t)m * N + j] = v;
+    }
+}
+
+// C[M][K] = (D[M][N] W[N][K]) (1 - H^2), N <= kNarrow: a thread keeps its
+// column of W over its rows
+__global__ void __launch_bounds__(256)
+    mlp_back_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
+                           const float *__restrict__ W, const float *__restrict__ H,
+                           float *__restrict__ C) {
+  for (int k = blockIdx.x * 256 + threadIdx.x; k < K; k += gridDim.x * 256) {
+    float w[kNarrow];
+#pragma unroll
+    for (int j = 0; j < kNarrow; j++) w[j] = j < N ? W[(int64_t)j * K + k] : 0.f;
+#pragma unroll 4
+    for (int m = blockIdx.y; m < M; m += gridDim.y) {
+      const float h = H[(int64_t)m * K + k];
+      float s = 0.f;
+#pragma unroll
+      for (int j = 0; j < kNarrow; j++)
+        if (j < N) s = fmaf(__ldg(D + (int64_t)m * N + j), w[j], s);
+      C[(int64_t)m * K + k] = s * (1.f - h * h);
     }
   }
 }
 
-// C[M][N] = A[M][K] * B[K][N]   (dH = dZ W)
+// Split blockIdx.y of dW[N][K] = D^T X and of the sums of D where D or X
+// (wide_is_d) has at most kNarrow columns: a thread per column of the wide
+// one, four groups of rows a block, 32 rows of the narrow one at a time in
+// shared memory (4096 rows, 256 x 8: 5 us, 21 us as tiles and column sums).
 __global__ void __launch_bounds__(256)
-    gemm_xw_kernel(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B,
-                   float *__restrict__ C) {
-  __shared__ float As[TK][TM + 4];
-  __shared__ float Bs[TK][TN + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    for (int t = threadIdx.x; t < TM * TK; t += 256) {
-      const int mm = t / TK, kk = t % TK;
-      const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? A[(int64_t)gm * K + gk] : 0.f;
-      const int kb = t / TN, nb = t % TN;
-      const int gkb = k0 + kb, gnb = n0 + nb;
-      Bs[kb][nb] = (gkb < K && gnb < N) ? B[(int64_t)gkb * N + gnb] : 0.f;
+    mlp_grad_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
+                           const float *__restrict__ X, float *__restrict__ G, int mchunk,
+                           int wide_is_d) {
+  constexpr int R = 32;
+  __shared__ __align__(16) float q[4][R][kNarrow];
+  __shared__ float red[4][kNarrow + 1][64];
+  const int c = threadIdx.x & 63, grp = threadIdx.x >> 6, i = blockIdx.x * 64 + c;
+  const int nw = wide_is_d ? N : K, nn = wide_is_d ? K : N;
+  const float *P = wide_is_d ? D : X, *Q = wide_is_d ? X : D;
+  const int per = (mchunk + 3) / 4, b0 = blockIdx.y * mchunk;
+  const int mb = b0 + grp * per, me = min(min(M, b0 + mchunk), mb + per);
+  G += (int64_t)blockIdx.y * ((int64_t)N * K + N);
+  float s[kNarrow] = {}, sd = 0.f;
+  for (int r0 = 0; r0 < per; r0 += R) {
+    __syncthreads();
+    for (int t = c; t < R * kNarrow; t += 64) {
+      const int m = mb + r0 + t / kNarrow, j = t % kNarrow;
+      q[grp][t / kNarrow][j] = m < me && j < nn ? Q[(int64_t)m * nn + j] : 0.f;
     }
     __syncthreads();
+    if (i >= nw) continue;
+    const float *p = P + (int64_t)(mb + r0) * nw + i;
+    auto add = [&](int r, float x) {
+      const float4 u = *reinterpret_cast<const float4 *>(&q[grp][r][0]);
+      const float4 v = *reinterpret_cast<const float4 *>(&q[grp][r][4]);
+      const float y[kNarrow] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int kk = 0; kk < TK; kk++) {
-      float a[4], b[4];
+      for (int j = 0; j < kNarrow; j++) s[j] = fmaf(x, y[j], s[j]);
+      sd += wide_is_d ? x : q[grp][r][c & (kNarrow - 1)];
+    };
+    if (mb + r0 + R <= me) {  // 16 loads in flight; under a condition one
+      for (int r = 0; r < R; r += 16) {
+        float x[16];
 #pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
+        for (int t = 0; t < 16; t++) x[t] = p[(int64_t)(r + t) * nw];
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn < N) C[(int64_t)gm * N + gn] = acc[i][j];
+        for (int t = 0; t < 16; t++) add(r + t, x[t]);
+      }
+    } else {
+      for (int r = 0; mb + r0 + r < me; r++) add(r, p[(int64_t)r * nw]);
     }
   }
+#pragma unroll
+  for (int j = 0; j < kNarrow; j++) red[grp][j][c] = s[j];
+  red[grp][kNarrow][c] = sd;
+  __syncthreads();
+  if (grp != 0 || i >= nw) return;
+#pragma unroll
+  for (int j = 0; j < kNarrow; j++) {
+    if (j >= nn) break;
+    const float v = (red[0][j][c] + red[1][j][c]) + (red[2][j][c] + red[3][j][c]);
+    G[wide_is_d ? (int64_t)i * K + j : (int64_t)j * K + i] = v;
+  }
+  if (i < N)
+    G[(int64_t)N * K + i] = (red[0][kNarrow][c] + red[1][kNarrow][c]) +
+                            (red[2][kNarrow][c] + red[3][kNarrow][c]);
 }
 
-// G[N][K] = D^T[N][M] * X[M][K]  (weight gradient dW = dZ^T H).  The batch
-// M is split over blockIdx.z in chunks of mchunk rows; split z writes its
-// partial sum to G + z N K (reduce_splits_kernel adds them in a fixed
-// order, so the result is deterministic).
-__global__ void __launch_bounds__(256)
-    gemm_dTx_kernel(int M, int N, int K, const float *__restrict__ D, const float *__restrict__ X,
-                    float *__restrict__ G, int mchunk) {
-  __shared__ float Ds[TK][TM + 4];
-  __shared__ float Xs[TK][TN + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int n0 = blockIdx.y * TM, k0c = blockIdx.x * TN;
-  const int mb = blockIdx.z * mchunk, me = min(M, mb + mchunk);
-  G += (int64_t)blockIdx.z * N * K;
-  float acc[4][4] = {};
-  for (int m0 = mb; m0 < me; m0 += TK) {
-    for (int t = threadIdx.x; t < TM * TK; t += 256) {
-      const int mm = t / TM, nn = t % TM;
-      const int gm = m0 + mm;
-      Ds[mm][nn] = (gm < me && n0 + nn < N) ? D[(int64_t)gm * N + n0 + nn] : 0.f;
-      Xs[mm][nn] = (gm < me && k0c + nn < K) ? X[(int64_t)gm * K + k0c + nn] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int mm = 0; mm < TK; mm++) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = Ds[mm][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Xs[mm][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+// aligned for the 16-byte loads of tile_load
+static bool vec4(const float *p, int ld) { return (ld & 3) == 0 && ((uintptr_t)p & 15) == 0; }
+
+// act(X W^T + b) of one layer
+static void launch_layer(const float *X, int B, int K, int N, const float *W, const float *b,
+                         float *Y, int act, cudaStream_t st) {
+  if (N <= kNarrow) {
+    mlp_forward_narrow_kernel<<<(B + 7) / 8, 256, 0, st>>>(B, N, K, X, W, b, Y, act);
+    return;
   }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int gn = n0 + ty * 4 + i;
-    if (gn >= N) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int gk = k0c + tx * 4 + j;
-      if (gk < K) G[(int64_t)gn * K + gk] = acc[i][j];
-    }
-  }
+  dim3 grid((N + TN - 1) / TN, (B + TM - 1) / TM);
+  mlp_gemm_kernel<MLP_FORWARD><<<grid, 256, 0, st>>>(B, N, K, X, W, b, Y, act, 0, vec4(X, K),
+                                                     vec4(W, K), vec4(Y, N));
 }
 
 // g[i] = sum over the splits z (in order) of P[z][i]
-__global__ void reduce_splits_kernel(int nsplit, int n, const float *__restrict__ P,
-                                     float *__restrict__ g) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int z = 0; z < nsplit; z++) s += P[(int64_t)z * n + i];
-    g[i] = s;
-  }
-}
-
-// column sums of D[M][N] -> g[N] (bias gradient), one block per column tile
-__global__ void colsum_kernel(int M, int N, const float *__restrict__ D, float *__restrict__ g) {
-  __shared__ float sh[256];
-  const int n = blockIdx.x;
+__global__ void grad_sum_kernel(int nsplit, int n, const float *__restrict__ P,
+                                float *__restrict__ g) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
   float s = 0.f;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) s += D[(int64_t)m * N + n];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) g[n] = sh[0];
+#pragma unroll 8
+  for (int z = 0; z < nsplit; z++) s += P[(int64_t)z * n + i];
+  g[i] = s;
 }
 
 // dY = 2 mask (Y - T) / msum ; per-block partial of sum mask (Y-T)^2
@@ -217,13 +437,6 @@ __global__ void loss_grad_kernel(int n, const float *__restrict__ Y, const float
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// dZ = dH * (1 - H^2)
-__global__ void tanh_back_kernel(int64_t n, const float *__restrict__ H, float *__restrict__ d) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    d[i] *= 1.f - H[i] * H[i];
-}
-
 __global__ void adam_kernel(int n, float *__restrict__ w, const float *__restrict__ g,
                             float *__restrict__ m, float *__restrict__ v, float lr, float b1,
                             float b2, float eps, float c1, float c2) {
@@ -237,12 +450,22 @@ __global__ void adam_kernel(int n, float *__restrict__ w, const float *__restric
   }
 }
 
-// gather rows idx[b] of X[n][k] -> Xb[b][k]
-__global__ void gather_rows_kernel(int B, int k, const int *__restrict__ idx,
-                                   const float *__restrict__ X, float *__restrict__ Xb) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < B * k; t += gridDim.x * blockDim.x) {
-    const int b = t / k, j = t - b * k;
-    Xb[t] = X[(int64_t)idx[b] * k + j];
+// rows idx[b] of X[n][ni], T[n][no] and K[n][no] -> Xb, Tb, Kb
+__global__ void gather_rows_kernel(int B, int ni, int no, const int *__restrict__ idx,
+                                   const float *__restrict__ X, const float *__restrict__ T,
+                                   const float *__restrict__ K, float *__restrict__ Xb,
+                                   float *__restrict__ Tb, float *__restrict__ Kb) {
+  const int64_t w = ni + 2 * no;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < B * w;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = t / w, r = idx[b];
+    const int j = (int)(t - b * w);
+    if (j < ni)
+      Xb[b * ni + j] = X[r * ni + j];
+    else if (j < ni + no)
+      Tb[b * no + j - ni] = T[r * no + j - ni];
+    else
+      Kb[b * no + j - ni - no] = K[r * no + j - ni - no];
   }
 }
 
@@ -256,7 +479,7 @@ struct Mlp {
   float *d_dA = nullptr, *d_dB = nullptr;  // backward scratch [cap][maxw]
   float *d_part = nullptr, *h_part = nullptr;
   float *d_xb = nullptr, *d_tb = nullptr, *d_mb = nullptr;
-  float *d_split = nullptr;          // weight-gradient partial sums [kMaxSplit][maxw][maxw]
+  float *d_split = nullptr;          // gradient partial sums [kMaxSplit][maxw * (maxw + 1)]
   int *d_idx = nullptr;
   int adam_t = 0;
   int dev = 0;                       // the device the network lives on
@@ -310,7 +533,7 @@ struct Mlp {
         cudaMalloc(&d_idx, sizeof(int) * (size_t)B) != cudaSuccess)
       return fail("MLP scratch");
     if (!d_split &&
-        cudaMalloc(&d_split, sizeof(float) * (size_t)kMaxSplit * maxw() * maxw()) != cudaSuccess)
+        cudaMalloc(&d_split, sizeof(float) * (size_t)kMaxSplit * maxw() * (maxw() + 1)) != cudaSuccess)
       return fail("MLP scratch");
     cap = B;
     return 0;
@@ -318,10 +541,8 @@ struct Mlp {
   void forward(const float *X, int B) {
     const float *in = X;
     for (int l = 0; l < layers(); l++) {
-      const int K = width[l], N = width[l + 1];
-      dim3 grid((N + TN - 1) / TN, (B + TM - 1) / TM);
-      gemm_xwT_kernel<<<grid, 256, 0, st>>>(B, N, K, in, d_w + woff[l], d_w + boff[l], act[l],
-                                            l + 1 < layers() ? 1 : 0);
+      launch_layer(in, B, width[l], width[l + 1], d_w + woff[l], d_w + boff[l], act[l],
+                   l + 1 < layers() ? 1 : 0, st);
       in = act[l];
     }
   }
@@ -335,24 +556,37 @@ struct Mlp {
     for (int l = nl - 1; l >= 0; l--) {
       const int K = width[l], N = width[l + 1];
       const float *Hin = l == 0 ? X : act[l - 1];
-      // dW_l = dZ^T Hin  [N][K], the batch split over up to kMaxSplit CTA
-      // layers so that the grid covers the GPU; db_l = colsum dZ
+      // dW_l = dZ^T Hin  [N][K] and db_l = colsum dZ, which follows it in
+      // d_g; the batch split over up to kMaxSplit CTA layers so that the grid
+      // covers the GPU
       const int nsplit = std::max(1, std::min(kMaxSplit, B / 128));
       const int mchunk = ((B + nsplit - 1) / nsplit + TK - 1) / TK * TK;
-      dim3 g1((K + TN - 1) / TN, (N + TM - 1) / TM, nsplit);
-      if (nsplit == 1) {
-        gemm_dTx_kernel<<<g1, 256, 0, st>>>(B, N, K, dcur, Hin, d_g + woff[l], mchunk);
+      float *part = nsplit == 1 ? d_g + woff[l] : d_split;
+      if (K <= kNarrow || N <= kNarrow) {
+        const int wide_is_d = K <= kNarrow;
+        dim3 g1(((wide_is_d ? N : K) + 63) / 64, nsplit);
+        mlp_grad_narrow_kernel<<<g1, 256, 0, st>>>(B, N, K, dcur, Hin, part, mchunk, wide_is_d);
       } else {
-        gemm_dTx_kernel<<<g1, 256, 0, st>>>(B, N, K, dcur, Hin, d_split, mchunk);
-        reduce_splits_kernel<<<(N * K + 255) / 256, 256, 0, st>>>(nsplit, N * K, d_split,
-                                                                  d_g + woff[l]);
+        dim3 g1((K + TN - 1) / TN, (N + TM - 1) / TM, nsplit);
+        mlp_gemm_kernel<MLP_GRAD><<<g1, 256, 0, st>>>(N, K, B, dcur, Hin, nullptr, part, 0,
+                                                      mchunk, vec4(dcur, N), vec4(Hin, K),
+                                                      vec4(part, K) && (nsplit == 1 || (N & 3) == 0));
       }
-      colsum_kernel<<<N, 256, 0, st>>>(B, N, dcur, d_g + boff[l]);
+      if (nsplit > 1)
+        grad_sum_kernel<<<(N * K + N + 255) / 256, 256, 0, st>>>(nsplit, N * K + N, d_split,
+                                                                 d_g + woff[l]);
       if (l == 0) break;
-      // dH_{l-1} = dZ W_l  [B][K]; dZ_{l-1} = dH * (1 - H^2)
-      dim3 g2((K + TN - 1) / TN, (B + TM - 1) / TM);
-      gemm_xw_kernel<<<g2, 256, 0, st>>>(B, K, N, dcur, d_w + woff[l], dnext);
-      tanh_back_kernel<<<304, 256, 0, st>>>((int64_t)B * K, act[l - 1], dnext);
+      // dZ_{l-1} = (dZ W_l) (1 - H^2)  [B][K]
+      const float *W = d_w + woff[l];
+      if (N <= kNarrow) {
+        dim3 g2((K + 255) / 256, std::min(B, 1216));
+        mlp_back_narrow_kernel<<<g2, 256, 0, st>>>(B, N, K, dcur, W, act[l - 1], dnext);
+      } else {
+        dim3 g2((K + TN - 1) / TN, (B + TM - 1) / TM);
+        mlp_gemm_kernel<MLP_BACK><<<g2, 256, 0, st>>>(B, K, N, dcur, W, act[l - 1], dnext, 0, 0,
+                                                      vec4(dcur, N), vec4(W, K),
+                                                      vec4(dnext, K) && vec4(act[l - 1], K));
+      }
       float *t = dcur;
       dcur = dnext;
       dnext = t;
@@ -527,9 +761,8 @@ int gb_mlp_train_device(gb_mlp *m, const float *d_x, const float *d_t, const flo
     if (ms <= 0.0) continue;
     e = cudaMemcpyAsync(M.d_idx, idx.data(), sizeof(int) * B, cudaMemcpyHostToDevice, M.st);
     if (e != cudaSuccess) return gb::cuda_fail(e, "batch");
-    gb::gather_rows_kernel<<<304, 256, 0, M.st>>>(B, ni, M.d_idx, d_x, M.d_xb);
-    gb::gather_rows_kernel<<<304, 256, 0, M.st>>>(B, no, M.d_idx, d_t, M.d_tb);
-    gb::gather_rows_kernel<<<304, 256, 0, M.st>>>(B, no, M.d_idx, d_mask, M.d_mb);
+    gb::gather_rows_kernel<<<304, 256, 0, M.st>>>(B, ni, no, M.d_idx, d_x, d_t, d_mask, M.d_xb,
+                                                  M.d_tb, M.d_mb);
     M.forward(M.d_xb, B);
     // the loss is read back on the last step only: no per-step host wait
     if (M.backward(M.d_xb, M.d_tb, M.d_mb, B, (float)ms, s + 1 == steps ? &loss : nullptr))
@@ -622,9 +855,8 @@ extern "C" int gb_mlp_forward_noalloc(gb_mlp *m, const float *d_x, int B, float 
   for (int l = 0; l < L; l++) {
     const int K = M.width[l], N = M.width[l + 1];
     float *out = l + 1 == L ? d_y : buf[l & 1];
-    dim3 grid((N + gb::TN - 1) / gb::TN, (B + gb::TM - 1) / gb::TM);
-    gb::gemm_xwT_kernel<<<grid, 256, 0, cs>>>(B, N, K, in, M.d_w + M.woff[l], M.d_w + M.boff[l],
-                                              out, l + 1 < L ? 1 : 0);
+    gb::launch_layer(in, B, K, N, M.d_w + M.woff[l], M.d_w + M.boff[l], out, l + 1 < L ? 1 : 0,
+                     cs);
     in = out;
   }
   e = cudaGetLastError();
