@@ -650,6 +650,7 @@ Solver::~Solver() {
   line_lo.release();
   line_up.release();
   if (h_work) cudaFreeHost(h_work);
+  if (ev_h) cudaEventDestroy(ev_h);
   if (h_segout) cudaFreeHost(h_segout);
 }
 
@@ -828,6 +829,7 @@ int Solver::init(Context *c, int krylov) {
   GB_CU(cudaMalloc(&d_scale, sizeof(double) * N), "scale");
   const size_t wk = (size_t)(kRedBlocks * 3 + (krylov + 2) * kGsBlocks + 4 * (krylov + 2) + 96);
   GB_CU(cudaMalloc(&d_work, sizeof(double) * wk), "work");
+  if (!ev_h) GB_CU(cudaEventCreateWithFlags(&ev_h, cudaEventDisableTiming), "event");
   GB_CU(cudaMallocHost(&h_work, sizeof(double) * 4 * (krylov + 2) + 64 * sizeof(double)), "host");
   GB_CU(cudaMalloc(&d_V, sizeof(double) * (size_t)(krylov + 1) * N), "Krylov basis");
   GB_CU(cudaMalloc(&d_t, sizeof(double) * N), "t");
@@ -1173,22 +1175,33 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     basis_vector(V, 0, nullptr, dh, V);
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
-    int j = 0;
-    bool done = false;
-    for (; j < m && total < maxit; j++) {
-      const T *zj = t;  // M^-1 v_j
+    // w = A M^-1 v_k
+    auto apply_operator = [&](int k) -> int {
+      const T *z = t;  // M^-1 v_k
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
-          // the preconditioner in FP32, z_j kept in FP64
+          // the preconditioner in FP32, z_k kept in FP64
           if (S.apply_prec32(st)) return -1;
-          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + j * ld);
-          zj = S.d_Z + j * ld;
+          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
+          z = S.d_Z + k * ld;
         }
       }
       if (!flexible) {
         if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
       }
-      GB_CU(spmv<T>(C, lpr, A, zj, w, st), "spmv");
+      GB_CU(spmv<T>(C, lpr, A, z, w, st), "spmv");
+      return 0;
+    };
+    int j = 0;
+    bool done = false;
+    // the operator on v_j is queued before the host has seen step j - 1,
+    // unless the residual's last decrease says that the step will be the last
+    // one; queued after, the GPU waited 4 to 10 us a step for the copy, the
+    // rotations and the launches (1 to 2 % of a solve)
+    bool ahead = false;
+    double before = HUGE_VAL;  // residual a step earlier
+    for (; j < m && total < maxit; j++) {
+      if (!ahead && apply_operator(j)) return -1;
       // CGS2 on the device; the host reads both passes and the norm in one copy
       std::vector<double> hcol(j + 2, 0.0);
       double *dh1 = dh, *dh2 = dh + (m + 2), *dnrm = dh + 2 * (m + 2);
@@ -1201,7 +1214,12 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
       GB_CU(cudaGetLastError(), "Arnoldi step");
       GB_CU(cudaMemcpyAsync(hh, dh, sizeof(double) * (2 * (m + 2) + 1), cudaMemcpyDeviceToHost,
                             st), "h");
-      GB_CU(cudaStreamSynchronize(st), "h sync");
+      GB_CU(cudaEventRecord(S.ev_h, st), "h");
+      const double now = std::fabs(g[j]);
+      ahead = j + 1 < m && total + 1 < maxit && now * std::fmin(1.0, now / before) > tol * bnorm;
+      before = now;
+      if (ahead && apply_operator(j + 1)) return -1;
+      GB_CU(cudaEventSynchronize(S.ev_h), "h sync");
       for (int i = 0; i <= j; i++) hcol[i] = hh[i] + hh[(m + 2) + i];
       const double hn = hh[2 * (m + 2)];
       hcol[j + 1] = hn;
@@ -1460,21 +1478,28 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
       done[sg] = active[sg] ? 0 : -1;  // -1: converged before this cycle
       used[sg] = 0;
     }
-    int j = 0;
-    for (; j < m && total < maxit; j++) {
-      const T *zj = t;  // M^-1 v_j
+    // w = A M^-1 v_k
+    auto apply_operator = [&](int k) -> int {
+      const T *z = t;  // M^-1 v_k
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
-          // the (block-diagonal) preconditioner in FP32, z_j kept in FP64
+          // the (block-diagonal) preconditioner in FP32, z_k kept in FP64
           if (S.apply_prec32(st)) return -1;
-          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + j * ld);
-          zj = S.d_Z + j * ld;
+          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
+          z = S.d_Z + k * ld;
         }
       }
       if (!flexible) {
         if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
       }
-      GB_CU(spmv<T>(C, lpr, A, zj, w, st), "spmv");
+      GB_CU(spmv<T>(C, lpr, A, z, w, st), "spmv");
+      return 0;
+    };
+    int j = 0;
+    bool ahead = false;  // as in gmres
+    double before = HUGE_VAL;
+    for (; j < m && total < maxit; j++) {
+      if (!ahead && apply_operator(j)) return -1;
       seg_gs_kernel<T, GS_DOTS><<<nt, 256, 0, st>>>(j + 1, V, ld, nullptr, w, S.d_tile_seg,
                                                     S.d_tile_beg, S.d_tile_end, S.d_segpart);
       reduce(j + 1, o1);
@@ -1488,7 +1513,15 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
       GB_CU(cudaGetLastError(), "batched Arnoldi step");
       GB_CU(cudaMemcpyAsync(h1, o1, sizeof(double) * 3 * 32 * ns, cudaMemcpyDeviceToHost, st),
             "h");
-      GB_CU(cudaStreamSynchronize(st), "h sync");
+      GB_CU(cudaEventRecord(S.ev_h, st), "h");
+      double now = 0.0;  // the largest residual over its tolerance
+      for (int sg = 0; sg < ns; sg++)
+        if (done[sg] == 0)
+          now = std::fmax(now, std::fabs(g[(size_t)sg * (m + 1) + j]) / (tol * bnorm[sg]));
+      ahead = j + 1 < m && total + 1 < maxit && now * std::fmin(1.0, now / before) > 1.0;
+      before = now;
+      if (ahead && apply_operator(j + 1)) return -1;
+      GB_CU(cudaEventSynchronize(S.ev_h), "h sync");
       total++;
       bool changed = false, all_done = true;
       for (int sg = 0; sg < ns; sg++) {

@@ -88,6 +88,7 @@ struct Solver {
   double *d_scale = nullptr;
   double *d_work = nullptr;     // reduction scratch
   double *h_work = nullptr;     // pinned host mirror
+  cudaEvent_t ev_h = nullptr;   // an Arnoldi step's coefficients are on the host
   int max_krylov = 0;
   double *d_V = nullptr;        // (m+1) x N Krylov basis (FP64)
   float *d_V32 = nullptr;       // (m+1) x N Krylov basis (FP32)
