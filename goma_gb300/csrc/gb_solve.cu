@@ -403,23 +403,63 @@ __global__ void to_f64_kernel(int64_t n, const float *__restrict__ x, double *__
 
 // ------------------------------------------------------------ SpMV
 
-// y = A x, LPR lanes per row (LPR divides 32)
-template <class T, int LPR>
-__global__ void spmv_kernel(int N, const int64_t *__restrict__ rowptr,
-                            const int *__restrict__ colidx, const T *__restrict__ vals,
-                            const T *__restrict__ x, T *__restrict__ y) {
-  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
-  const int l = threadIdx.x % LPR;
-  const bool live = g < N;  // the whole warp takes part in the shuffles
+// y = A x, LPR lanes for a group of up to four rows with the same columns:
+// the rows of a node (its energy row lacks the pressure columns and is a
+// group by itself).  One index and one gathered x serve all rows of a group,
+// and the rows' sums share the steps of the reduction: each halves the lanes
+// that keep a sum, 4 adds instead of 12 for four rows by 8 lanes.  A row's
+// products are added as by 8 lanes of its own.
+//
+// Bound in FP64 by the FP64 pipe (N = 160K, 34 M entries: 58 us of products
+// at 2 a clock and SM) about as much as by HBM (51 us): 82 us, 103 us a row at
+// a time.  Groups are sorted by rows and length: vertex nodes have rows five
+// times as long as centroids, and a warp takes as long as its longest (105 us
+// unsorted), as the launch does, so the longest come first.
+template <class T, int LPR, int ROWS>
+__device__ __forceinline__ void spmv_group(int64_t r0, int64_t len, int l,
+                                           const int *__restrict__ colidx,
+                                           const T *__restrict__ vals, const T *__restrict__ x,
+                                           acc_t<T> (&s)[4]) {
   using A = acc_t<T>;
-  A s = 0;
-  if (live) {
-    const int64_t r0 = rowptr[g], r1 = rowptr[g + 1];
-    for (int64_t k = r0 + l; k < r1; k += LPR) s = fmx((A)vals[k], (A)__ldg(x + colidx[k]), s);
-  }
+  const int *c = colidx + r0;
+  const T *v = vals + r0;
+#pragma unroll 4
+  for (int64_t k = l; k < len; k += LPR) {
+    const A xv = (A)__ldg(x + c[k]);
 #pragma unroll
-  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
-  if (live && l == 0) y[g] = (T)s;
+    for (int r = 0; r < ROWS; r++) s[r] = fmx((A)v[r * len + k], xv, s[r]);
+  }
+}
+
+template <class T, int LPR>
+__global__ void __launch_bounds__(256)
+    spmv_kernel(int ng, const int2 *__restrict__ groups, const int64_t *__restrict__ rowptr,
+                const int *__restrict__ colidx, const T *__restrict__ vals,
+                const T *__restrict__ x, T *__restrict__ y) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPR, l = threadIdx.x % LPR;
+  using A = acc_t<T>;
+  A s[4] = {};
+  int2 gr = make_int2(0, 0);  // first row, rows
+  if (g < ng) {  // the whole warp takes part in the shuffles
+    gr = groups[g];
+    const int64_t r0 = rowptr[gr.x], len = rowptr[gr.x + 1] - r0;
+    if (gr.y == 4)
+      spmv_group<T, LPR, 4>(r0, len, l, colidx, vals, x, s);
+    else if (gr.y == 3)
+      spmv_group<T, LPR, 3>(r0, len, l, colidx, vals, x, s);
+    else if (gr.y == 2)
+      spmv_group<T, LPR, 2>(r0, len, l, colidx, vals, x, s);
+    else
+      spmv_group<T, LPR, 1>(r0, len, l, colidx, vals, x, s);
+  }
+  const bool hi = l & (LPR / 2), odd = l & (LPR / 4);
+  const A a = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], LPR / 2, LPR);
+  const A b = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], LPR / 2, LPR);
+  A t = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, LPR / 4, LPR);
+#pragma unroll
+  for (int o = LPR / 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o, LPR);
+  const int r = (hi ? 2 : 0) + (odd ? 1 : 0);
+  if (l % (LPR / 4) == 0 && r < gr.y) y[gr.x + r] = (T)t;
 }
 
 // ------------------------------------------------------------ ILU(0)
@@ -702,6 +742,35 @@ int Solver::init(Context *c, int krylov) {
   }
   GB_CU(cudaMalloc(&d_diag, sizeof(int64_t) * N), "diag");
   GB_CU(cudaMemcpy(d_diag, diag.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice), "diag");
+  // row groups of the products (spmv_kernel), most rows and longest rows first
+  {
+    // (a counting sort: the rows of one length in the order of the nodes)
+    int64_t longest = 0;
+    for (int i = 0; i < N; i++) longest = std::max(longest, L.rowptr[i + 1] - L.rowptr[i]);
+    auto each = [&](auto &&f) {
+      for (int n = 0; n < L.num_nodes; n++) {
+        const int f0 = L.fu[n], nr = L.fu[n + 1] - f0;
+        const int tr = L.energy && nr > L.dim ? L.dim : nr;  // the energy row
+        const int at[4] = {0, tr, std::min(tr + 1, nr), nr};
+        for (int p = 0; p < 3; p++)
+          for (int a = at[p]; a < at[p + 1]; a += 4) {
+            const int i = f0 + a, rows = std::min(4, at[p + 1] - a);
+            f(make_int2(i, rows),
+              (size_t)((4 - rows) * (longest + 1) + longest - (L.rowptr[i + 1] - L.rowptr[i])));
+          }
+      }
+    };
+    std::vector<int> start(4 * (longest + 1) + 1, 0);
+    each([&](int2, size_t key) { start[key + 1]++; });
+    for (size_t k = 1; k < start.size(); k++) start[k] += start[k - 1];
+    std::vector<int2> all(start.back());
+    each([&](int2 g, size_t key) { all[start[key]++] = g; });
+    nrowgrp = (int)all.size();
+    GB_CU(cudaMalloc(&d_rowgrp, sizeof(int2) * all.size()), "row groups");
+    owned.push_back(d_rowgrp);
+    GB_CU(cudaMemcpy(d_rowgrp, all.data(), sizeof(int2) * all.size(), cudaMemcpyHostToDevice),
+          "row groups");
+  }
   ordering = c->ilu_ordering;
   Layout Lp;
   const Layout *LP = &L;  // the layout the factors live in
@@ -890,16 +959,21 @@ static int lanes_per_row(const Layout &L) {
 
 template <class T>
 static cudaError_t spmv(const Context *C, int lpr, const T *vals, const T *x, T *y, cudaStream_t st) {
-  // FP64: 8 lanes a row.  On GB300 the FP64 product is bound by the FP64
-  // pipe as much as by HBM (ncu: pipe 89 % busy at 32 lanes a row, half of it
-  // the shuffle-reduction adds); 8 lanes cut those adds to a sixth.
-  if (sizeof(T) == 8) lpr = 8;
-  const int N = C->L.N, threads = 256;
-  const int blocks = (int)(((int64_t)N * lpr + threads - 1) / threads);
+  const Solver &S = *C->solver;
+  const int ng = S.nrowgrp, threads = 256;
+  // FP64: 8 lanes a group, few adds in the sums (N = 160K: 82 us, 95 us by 16
+  // lanes); 16 where that would not fill the chip twice and rows are long, so
+  // that the longest, 500 entries, would end alone (N = 50K: 38 us, 52 us by 8
+  // lanes; short 2-D rows: 7.5 us by 8, 8.4 us by 16)
+  if (sizeof(T) == 8)
+    lpr = (int64_t)ng * 8 < 2 * (int64_t)C->num_sms * 1536 && C->L.nnz >= 96 * (int64_t)C->L.N
+              ? 16
+              : 8;
+  const int blocks = (int)(((int64_t)ng * lpr + threads - 1) / threads);
   switch (lpr) {
-  case 32: spmv_kernel<T, 32><<<blocks, threads, 0, st>>>(N, C->d_rowptr, C->d_colidx, vals, x, y); break;
-  case 16: spmv_kernel<T, 16><<<blocks, threads, 0, st>>>(N, C->d_rowptr, C->d_colidx, vals, x, y); break;
-  default: spmv_kernel<T, 8><<<blocks, threads, 0, st>>>(N, C->d_rowptr, C->d_colidx, vals, x, y);
+  case 32: spmv_kernel<T, 32><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
+  case 16: spmv_kernel<T, 16><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
+  default: spmv_kernel<T, 8><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y);
   }
   return cudaGetLastError();
 }

@@ -88,6 +88,8 @@ struct Solver {
   double *d_scale = nullptr;
   double *d_work = nullptr;     // reduction scratch
   double *h_work = nullptr;     // pinned host mirror
+  int2 *d_rowgrp = nullptr;     // rows with the same columns: first row, rows (at most 4)
+  int nrowgrp = 0;
   cudaEvent_t ev_h = nullptr;   // an Arnoldi step's coefficients are on the host
   int max_krylov = 0;
   double *d_V = nullptr;        // (m+1) x N Krylov basis (FP64)

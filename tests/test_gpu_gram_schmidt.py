@@ -1,4 +1,6 @@
-"""The Gram-Schmidt kernels of the Krylov solvers where their tiles end: fewer
+"""The Gram-Schmidt kernels of the Krylov solvers where their tiles end, and the
+product with the matrix in all its groups of rows (one to four rows, 8 and 16
+lanes): fewer
 unknowns than one tile of 128 rows, a few rows past a tile, more tiles than
 blocks, Krylov spaces of 1, 3, 4 and 5 vectors around the four columns that a
 warp takes at once and of 37 around the 32 of a block, independent problems
@@ -28,6 +30,8 @@ CASES = {
     "cavity 9x4": lambda: cavity(9, 4),
     "cube 4x2x3": lambda: cube(4, 2, 3),
     "cavity 130x70": lambda: cavity(130, 70),
+    "reacting 2x2x2": lambda: pb.reacting_channel_3d(2, 2, 2),
+    "bratu 5x5": lambda: pb.bratu_square_2d(5),
     "40 cavities 2x2": lambda: union(cavity(2, 2), 40),
     "3 cavities 20x17": lambda: union(cavity(20, 17), 3),
 }
