@@ -268,9 +268,12 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
-// out[j] = sum over the nblocks partial sums of column j, a block per column
+// out[j] = sum over the nblocks partial sums of column j, a block per column;
+// host[j] the same in page-locked memory, which the host reads after the
+// step: a copy in its place cost 10 us a step, most of it before and after
 __global__ void __launch_bounds__(128)
-    multidot_final_kernel(int nblocks, const double *__restrict__ part, double *__restrict__ out) {
+    multidot_final_kernel(int nblocks, const double *__restrict__ part, double *__restrict__ out,
+                          double *__restrict__ host) {
   __shared__ double red[4];
   const int j = blockIdx.x;
   double s = 0.0;
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(128)
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x == 0) out[j] = (red[0] + red[1]) + (red[2] + red[3]);
+  if (threadIdx.x == 0) out[j] = host[j] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // y = sum_j c[j] V[:, j]  (c on device)
@@ -295,12 +298,32 @@ __global__ void gemv_kernel(int N, int k, const T *__restrict__ V, int64_t ld,
   }
 }
 
-// y = x / norm (0 where the norm is 0), and the same to y2, the operand of the
-// preconditioner.  The norm: norm[0], or with nparts > 0 the root of the sum
-// of part[0..nparts), formed alike by every block and kept in norm[0].
+// What the preconditioner wants before it: its operand, where that is not the
+// basis vector itself, and outputs of the two sweeps without a value
+// (sync_free_apply); NULL where not wanted.
+template <class T2>
+struct SweepIo {
+  T2 *in = nullptr, *out1 = nullptr, *out2 = nullptr;
+  int *tickets = nullptr;  // of the two sweeps
+  __device__ __forceinline__ void put(int64_t i, T2 v) const {
+    if (in) in[i] = v;
+    if (out1) {
+      set_unpublished(out1 + i);
+      set_unpublished(out2 + i);
+    }
+  }
+  __device__ __forceinline__ void start() const {
+    if (tickets && blockIdx.x == 0 && threadIdx.x < 2) tickets[threadIdx.x] = 0;
+  }
+};
+
+// y = x / norm (0 where the norm is 0), and the sweeps' vectors.  The norm:
+// norm[0], or with nparts > 0 the root of the sum of part[0..nparts), formed
+// alike by every block and kept in norm[0] and in the host's host[0].
 template <class T, class T2>
 __global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *__restrict__ part,
-                                  double *norm, T *y, T2 *__restrict__ y2) {
+                                  double *norm, double *host, T *y, SweepIo<T2> io) {
+  io.start();
   using A = acc_t<T>;
   __shared__ double red[kRedThreads / 32];
   __shared__ double inv;
@@ -319,7 +342,7 @@ __global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *_
       nv = 0.0;
       for (int q = 0; q < kRedThreads / 32; q++) nv += red[q];
       nv = sqrt(nv);
-      if (blockIdx.x == 0) norm[0] = nv;
+      if (blockIdx.x == 0) norm[0] = host[0] = nv;
     } else {
       nv = norm[0];
     }
@@ -330,7 +353,7 @@ __global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *_
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     const T v = (T)((A)x[i] * a);
     y[i] = v;
-    if (y2) y2[i] = (T2)v;
+    io.put(i, (T2)v);
   }
 }
 
@@ -1089,13 +1112,12 @@ int Solver::copy_factors(double *host, bool fp32, cudaStream_t st) {
 }
 
 template <class T>
-static int sync_free_apply(Solver *S, T *z, cudaStream_t st) {
-  if (!S->d_sweep_y)
-    GB_CU(cudaMalloc(&S->d_sweep_y, sizeof(double) * (size_t)S->N), "trsv scratch");
+static int sync_free_apply(Solver *S, const T *in, T *z, cudaStream_t st) {
+  if (S->ensure_sweep_y()) return -1;
   T *y = static_cast<T *>(S->d_sweep_y);
   LineArgs a{};
   a.error = (int *)(S->d_flags + 4);
-  a.ticket = (int *)(S->d_flags + 8);
+  a.ticket = S->sweep_tickets();
   a.spin_limit = S->C->sweep_spin_limit > 0 ? S->C->sweep_spin_limit : kSpinLimit;
   const T *vl = sizeof(T) == 4 ? (const T *)S->d_line_lo32 : (const T *)S->d_line_lo;
   const T *vu = sizeof(T) == 4 ? (const T *)S->d_line_up32 : (const T *)S->d_line_up;
@@ -1103,16 +1125,46 @@ static int sync_free_apply(Solver *S, T *z, cudaStream_t st) {
   // reverse order (every dependency after its dependant) on one CTA, whose
   // first wait can then only end by running out
   const bool rev = S->C->sweep_reverse_lower != 0;
-  // L: z -> y, then U: y -> z; each output starts all unpublished
+  // L: in -> y, then U: y -> z; each output starts all unpublished
   const int prep = 2 * S->num_sms;
   a.lines = rev ? S->line_lo.d_lines_rev : S->line_lo.d_lines;
-  trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, y, a.ticket);
-  GB_CU(line_sweep<T>(S->line_lo, a, vl, z, y, S->num_sms, rev, st), "trsv");
+  if (in == z) trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, y, a.ticket);
+  GB_CU(line_sweep<T>(S->line_lo, a, vl, in, y, S->num_sms, rev, st), "trsv");
   a.lines = S->line_up.d_lines;
-  trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, z, a.ticket);
+  a.ticket++;
+  if (in == z) trsv_prepare_kernel<T><<<prep, 256, 0, st>>>(S->N, z, a.ticket);
   GB_CU(line_sweep<T>(S->line_up, a, vu, y, z, S->num_sms, false, st), "trsv");
   GB_CU(cudaGetLastError(), "trsv");
   return 0;
+}
+
+int Solver::ensure_sweep_y() {
+  if (!d_sweep_y)
+    GB_CU(cudaMalloc(&d_sweep_y, sizeof(double) * (size_t)N), "trsv scratch");
+  return 0;
+}
+
+bool Solver::direct_sweeps() const { return ordering != 1 && !use_level_graph(); }
+
+int *Solver::sweep_tickets() const { return (int *)(d_flags + 8); }
+
+// The vectors of the next operator application, for the kernel that writes
+// the basis vector: in direct sweeps the operand `in` stays apart from the
+// output z, so that this kernel can also clear both sweeps' outputs (a kernel
+// before each sweep took 6 us of the step).  T2 is the preconditioner's type;
+// own = false: the operand is the basis vector itself.
+template <class T2>
+static SweepIo<T2> sweep_io(const Solver &S, T2 *z, bool own) {
+  SweepIo<T2> io;
+  if (!S.direct_sweeps()) {
+    io.in = z;
+    return io;
+  }
+  io.in = own ? (T2 *)S.d_sweep_y + S.N : nullptr;  // FP32: its second half
+  io.out1 = (T2 *)S.d_sweep_y;
+  io.out2 = z;
+  io.tickets = S.sweep_tickets();
+  return io;
 }
 
 // The line sweeps are the faster ones on every schedule measured, short ones
@@ -1144,7 +1196,7 @@ static int apply_prec(Solver *S, T *t, T *tp, cudaGraphExec_t graph, cudaStream_
     z = tp;
   }
   if (!S->use_level_graph()) {
-    if (sync_free_apply<T>(S, z, st)) return -1;
+    if (sync_free_apply<T>(S, z, z, st)) return -1;
   } else {
     GB_CU(cudaGraphLaunch(graph, st), "ILU apply");
   }
@@ -1224,13 +1276,16 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     *out = hh[0];
     return 0;
   };
-  // v = src / norm, and the preconditioner's copy of it
+  if (S.direct_sweeps() && S.ensure_sweep_y()) return -1;
+  // v = src / norm, and what the preconditioner wants of it
   auto basis_vector = [&](const T *src, int nparts, const double *part, double *nrm, T *v) {
+    double *hn = hh + (nrm - dh);
     if (flexible)
-      scale_copy_kernel<T, float><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm,
-                                                                      v, S.d_t32);
+      scale_copy_kernel<T, float><<<kRedBlocks, kRedThreads, 0, st>>>(
+          N, src, nparts, part, nrm, hn, v, sweep_io(S, S.d_t32, true));
     else
-      scale_copy_kernel<T, T><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm, v, t);
+      scale_copy_kernel<T, T><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm, hn, v,
+                                                                  sweep_io(S, t, false));
   };
   GB_CU(cudaMemsetAsync(x, 0, sizeof(T) * N, st), "x0");
   double bnorm;
@@ -1252,16 +1307,21 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     // w = A M^-1 v_k
     auto apply_operator = [&](int k) -> int {
       const T *z = t;  // M^-1 v_k
+      const bool direct = S.direct_sweeps();
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
           // the preconditioner in FP32, z_k kept in FP64
-          if (S.apply_prec32(st)) return -1;
+          if (direct ? sync_free_apply<float>(&S, (float *)S.d_sweep_y + N, S.d_t32, st)
+                     : S.apply_prec32(st))
+            return -1;
           to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
           z = S.d_Z + k * ld;
         }
       }
       if (!flexible) {
-        if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
+        if (direct ? sync_free_apply<T>(&S, V + k * ld, t, st)
+                   : (f32 ? S.apply_prec32(st) : S.apply_prec64(st)))
+          return -1;
       }
       GB_CU(spmv<T>(C, lpr, A, z, w, st), "spmv");
       return 0;
@@ -1276,18 +1336,16 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
     double before = HUGE_VAL;  // residual a step earlier
     for (; j < m && total < maxit; j++) {
       if (!ahead && apply_operator(j)) return -1;
-      // CGS2 on the device; the host reads both passes and the norm in one copy
+      // CGS2 on the device; the host reads both passes and the norm in hh
       std::vector<double> hcol(j + 2, 0.0);
       double *dh1 = dh, *dh2 = dh + (m + 2), *dnrm = dh + 2 * (m + 2);
       gs_kernel<T, GS_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, nullptr, w, dpart);
-      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh1);
+      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh1, hh);
       gs_kernel<T, GS_SUB_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh1, w, dpart);
-      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh2);
+      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh2, hh + (m + 2));
       gs_kernel<T, GS_SUB_NORM><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh2, w, dpart);
       basis_vector(w, gs_blocks, dpart, dnrm, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "Arnoldi step");
-      GB_CU(cudaMemcpyAsync(hh, dh, sizeof(double) * (2 * (m + 2) + 1), cudaMemcpyDeviceToHost,
-                            st), "h");
       GB_CU(cudaEventRecord(S.ev_h, st), "h");
       const double now = std::fabs(g[j]);
       ahead = j + 1 < m && total + 1 < maxit && now * std::fmin(1.0, now / before) > tol * bnorm;
@@ -1428,16 +1486,18 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
-// out[s][j] = sum over the tiles of block s of part[t][j]; a warp per (s, j)
+// out[s][j] = sum over the tiles of block s of part[t][j], a warp per (s, j),
+// and the same to the host (multidot_final_kernel)
 __global__ void seg_reduce_kernel(int nseg, int k, const int *__restrict__ tptr,
-                                  const double *__restrict__ part, double *__restrict__ out) {
+                                  const double *__restrict__ part, double *__restrict__ out,
+                                  double *__restrict__ host) {
   const int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= nseg * k) return;
   const int sg = u / k, j = u - sg * k;
   double sum = 0.0;
   for (int t = tptr[sg] + lane; t < tptr[sg + 1]; t += 32) sum += part[(int64_t)t * 32 + j];
   sum = warp_sum(sum);
-  if (lane == 0) out[sg * 32 + j] = sum;
+  if (lane == 0) out[sg * 32 + j] = host[sg * 32 + j] = sum;
 }
 
 // y = sum_j c[s][j] V_j on block s
@@ -1460,13 +1520,13 @@ __global__ void seg_gemv_kernel(int k, const T *__restrict__ V, int64_t ld,
 }
 
 // dst = src * alpha[s] on block s; alpha = 1 / sqrt(norm2[s]) for active
-// blocks with a nonzero norm, else 0; the same to dst2, the operand of the
-// preconditioner
+// blocks with a nonzero norm, else 0; and the sweeps' vectors
 template <class T, class T2>
 __global__ void seg_scale_kernel(const T *src, const double *__restrict__ norm2,
                                  const int *__restrict__ active, const int *__restrict__ tseg,
                                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
-                                 T *dst, T2 *__restrict__ dst2) {
+                                 T *dst, SweepIo<T2> io) {
+  io.start();
   const int t = blockIdx.x, sg = tseg[t];
   __shared__ double inv;
   if (threadIdx.x == 0) {
@@ -1478,7 +1538,7 @@ __global__ void seg_scale_kernel(const T *src, const double *__restrict__ norm2,
   for (int64_t i = tbeg[t] + threadIdx.x; i < tend[t]; i += blockDim.x) {
     const T v = (T)((acc_t<T>)src[i] * a);
     dst[i] = v;
-    dst2[i] = (T2)v;
+    io.put(i, (T2)v);
   }
 }
 
@@ -1499,7 +1559,8 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
   double *o1 = S.d_segout, *o2 = o1 + 32 * ns, *o3 = o2 + 32 * ns;
   double *h1 = S.h_segout, *h2 = h1 + 32 * ns, *h3 = h2 + 32 * ns;
   auto reduce = [&](int k, double *out) {
-    seg_reduce_kernel<<<(ns * k + 7) / 8, 256, 0, st>>>(ns, k, S.d_tile_ptr, S.d_segpart, out);
+    seg_reduce_kernel<<<(ns * k + 7) / 8, 256, 0, st>>>(ns, k, S.d_tile_ptr, S.d_segpart, out,
+                                                        h1 + (out - o1));
   };
   // w . v on every block
   auto dot1 = [&](const T *v, T *wv, double *out) {
@@ -1507,14 +1568,17 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
                                                   S.d_tile_beg, S.d_tile_end, S.d_segpart);
     reduce(1, out);
   };
-  // v = src / norm per block, and the preconditioner's copy of it
+  if (S.direct_sweeps() && S.ensure_sweep_y()) return -1;
+  // v = src / norm per block, and what the preconditioner wants of it
   auto basis_vector = [&](const T *src, T *v) {
     if (flexible)
       seg_scale_kernel<T, float><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
-                                                     S.d_tile_beg, S.d_tile_end, v, S.d_t32);
+                                                     S.d_tile_beg, S.d_tile_end, v,
+                                                     sweep_io(S, S.d_t32, true));
     else
       seg_scale_kernel<T, T><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
-                                                 S.d_tile_beg, S.d_tile_end, v, t);
+                                                 S.d_tile_beg, S.d_tile_end, v,
+                                                 sweep_io(S, t, false));
   };
   std::vector<int> active(ns, 1), done(ns, 0);
   std::vector<double> bnorm(ns), beta(ns), coef(32 * (size_t)ns);
@@ -1529,7 +1593,6 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
   GB_CU(cudaMemsetAsync(x, 0, sizeof(T) * N, st), "x0");
   GB_CU(cudaMemcpyAsync(V, b, sizeof(T) * N, cudaMemcpyDeviceToDevice, st), "r0");
   dot1(V, V, o3);
-  GB_CU(cudaMemcpyAsync(h3, o3, sizeof(double) * 32 * ns, cudaMemcpyDeviceToHost, st), "norms");
   GB_CU(cudaStreamSynchronize(st), "norms");
   bool any = false;
   for (int sg = 0; sg < ns; sg++) {
@@ -1555,16 +1618,21 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
     // w = A M^-1 v_k
     auto apply_operator = [&](int k) -> int {
       const T *z = t;  // M^-1 v_k
+      const bool direct = S.direct_sweeps();
       if constexpr (std::is_same<T, double>::value) {
         if (flexible) {
           // the (block-diagonal) preconditioner in FP32, z_k kept in FP64
-          if (S.apply_prec32(st)) return -1;
+          if (direct ? sync_free_apply<float>(&S, (float *)S.d_sweep_y + N, S.d_t32, st)
+                     : S.apply_prec32(st))
+            return -1;
           to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
           z = S.d_Z + k * ld;
         }
       }
       if (!flexible) {
-        if (f32 ? S.apply_prec32(st) : S.apply_prec64(st)) return -1;
+        if (direct ? sync_free_apply<T>(&S, V + k * ld, t, st)
+                   : (f32 ? S.apply_prec32(st) : S.apply_prec64(st)))
+          return -1;
       }
       GB_CU(spmv<T>(C, lpr, A, z, w, st), "spmv");
       return 0;
@@ -1585,8 +1653,6 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
       reduce(1, o3);
       basis_vector(w, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "batched Arnoldi step");
-      GB_CU(cudaMemcpyAsync(h1, o1, sizeof(double) * 3 * 32 * ns, cudaMemcpyDeviceToHost, st),
-            "h");
       GB_CU(cudaEventRecord(S.ev_h, st), "h");
       double now = 0.0;  // the largest residual over its tolerance
       for (int sg = 0; sg < ns; sg++)
@@ -1669,7 +1735,6 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
     GB_CU(spmv<T>(C, lpr, A, x, V, st), "spmv");
     sub_from_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(N, b, V);
     dot1(V, V, o3);
-    GB_CU(cudaMemcpyAsync(h3, o3, sizeof(double) * 32 * ns, cudaMemcpyDeviceToHost, st), "norms");
     GB_CU(cudaStreamSynchronize(st), "norms");
     double worst = 0.0;
     bool all_conv = true;

@@ -98,11 +98,16 @@ struct Solver {
   float *d_t32 = nullptr, *d_w32 = nullptr;
   double *d_Z = nullptr;        // m x N preconditioned vectors (flexible GMRES)
   cudaGraphExec_t prec64 = nullptr, prec32 = nullptr;  // captured ILU solves on d_t / d_t32
-  unsigned *d_flags = nullptr;  // [4] error word, [8] next line to draw (sync-free sweeps)
+  unsigned *d_flags = nullptr;  // [4] error word, [8], [9] next line to draw (sync-free sweeps)
   void *d_sweep_y = nullptr;    // sync-free sweeps: the L sweep's output (N values)
   int num_sms = 0;
   int check_trsv_error();
   // level-scheduled sweeps from a captured graph (else the sync-free ones)
+  // the sweeps take the Krylov loop's vectors as they are (no permutation, no
+  // captured graph)
+  bool direct_sweeps() const;
+  int ensure_sweep_y();
+  int *sweep_tickets() const;  // of the lower and the upper sweep
   bool use_level_graph() const;
   ~Solver();
   int init(Context *c, int krylov);
