@@ -37,6 +37,7 @@
 #include <cstdint>
 
 #include "gb_device.h"
+#include "gb_launch.cuh"
 
 namespace gb {
 
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(NTH)
   static_assert(sizeof(S2Tables) % 8 == 0, "copied by doubles");
   for (int t = tid; t < (int)(sizeof(S2Tables) / 8); t += NTH)
     reinterpret_cast<double *>(&stb)[t] = reinterpret_cast<const double *>(gtb)[t];
+  dependent_begin();
   const MaterialDev M = A.mat;
   const int e0 = blockIdx.x * EPB;
   const int live = min(EPB, nelem - e0);
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(NTH)
 template <bool ENERGY, bool JAC>
 __global__ void __launch_bounds__(128)
     assemble_rows_kernel(AsmArgs A, S2Nodes nd, S2Scratch in) {
+  dependent_begin();
   using namespace s2;
   constexpr int NV = ENERGY ? 3 : 2, Tr = ENERGY ? 2 : -1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -566,7 +569,7 @@ static cudaError_t launch_elems(const AsmArgs &a, const S2Tables *tb, int nelem,
   auto k = assemble_2d_kernel<ENERGY, CARREAU, JAC, EPB, NTH>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  k<<<(nelem + EPB - 1) / EPB, NTH, sm, st>>>(a, tb, nelem, s);
+  launch_dependent(k, (nelem + EPB - 1) / EPB, NTH, sm, st, a, tb, nelem, s);
   return cudaGetLastError();
 }
 
@@ -587,7 +590,7 @@ static cudaError_t launch_2d(const AsmArgs &a, const S2Tables *tb, int nelem, co
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
   }
-  k<<<(nd.num_nodes + 3) / 4, 128, sm, st>>>(a, nd, s);
+  launch_dependent(k, (nd.num_nodes + 3) / 4, 128, sm, st, a, nd, s);
   return cudaGetLastError();
 }
 

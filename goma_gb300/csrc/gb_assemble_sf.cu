@@ -56,6 +56,7 @@
 #include <cstdint>
 
 #include "gb_device.h"
+#include "gb_launch.cuh"
 
 namespace gb {
 
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(sf::NT, 3)
     S.loc[t] = tb->loc[t];
   }
 
+  dependent_begin();
   for (int ei = blockIdx.x; ei < nelem; ei += gridDim.x) {
     const int e = elems[ei];
     const double rho_e = A.elem_rho ? A.elem_rho[e] : M.density;
@@ -574,7 +576,7 @@ static cudaError_t launch_sf_t(const AsmArgs &a, const SfTables *tb, const int *
   }
   const int grid = nelem < grid_cap ? nelem : grid_cap;
   if (grid <= 0) return cudaSuccess;
-  k<<<grid, sf::NT, sm, st>>>(a, tb, elems, nelem);
+  launch_dependent(k, grid, sf::NT, sm, st, a, tb, elems, nelem);
   return cudaGetLastError();
 }
 

@@ -30,6 +30,7 @@
 #include <cstdint>
 
 #include "gb_device.h"
+#include "gb_launch.cuh"
 #include "gb_element.cuh"
 
 namespace gb {
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(256, 2)
     return S.pS;
   };
 
+  dependent_begin();
   for (int ei = blockIdx.x; ei < nelem; ei += gridDim.x) {
     const int e = elems[ei];
     __syncthreads();  // the previous element is done with shared memory
@@ -694,7 +696,7 @@ static cudaError_t launch_species_sf(const AsmArgs &a, const SfTables *tb, const
   if (e != cudaSuccess) return e;
   const int grid = nelem < 2 * sms ? nelem : 2 * sms;
   if (grid <= 0) return cudaSuccess;
-  k<<<grid, 256, sm, st>>>(a, tb, elems, nelem);
+  launch_dependent(k, grid, 256, sm, st, a, tb, elems, nelem);
   return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@
 
 #include "../../include/gb_newton.h"
 #include "gb_context.h"
+#include "gb_launch.cuh"
 
 namespace gb {
 
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(256, 2)
     mlp_gemm_kernel(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B,
                     const float *__restrict__ E, float *__restrict__ C, int act, int kchunk,
                     bool vec_a, bool vec_b, bool vec_c) {
+  dependent_begin();
   constexpr bool AK = OP != MLP_GRAD, BK = OP == MLP_FORWARD;
   union Smem {
     float t[2][2][TK][TM];         // buffer, operand
@@ -285,6 +287,7 @@ __global__ void __launch_bounds__(256)
     mlp_forward_narrow_kernel(int M, int N, int K, const float *__restrict__ A,
                               const float *__restrict__ W, const float *__restrict__ bias,
                               float *__restrict__ C, int act) {
+  dependent_begin();
   const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m >= M) return;
   float s[kNarrow] = {};
@@ -312,6 +315,7 @@ __global__ void __launch_bounds__(256)
     mlp_back_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
                            const float *__restrict__ W, const float *__restrict__ H,
                            float *__restrict__ C) {
+  dependent_begin();
   for (int k = blockIdx.x * 256 + threadIdx.x; k < K; k += gridDim.x * 256) {
     float w[kNarrow];
 #pragma unroll
@@ -336,6 +340,7 @@ __global__ void __launch_bounds__(256)
     mlp_grad_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
                            const float *__restrict__ X, float *__restrict__ G, int mchunk,
                            int wide_is_d) {
+  dependent_begin();
   constexpr int R = 32;
   __shared__ __align__(16) float q[4][R][kNarrow];
   __shared__ float red[4][kNarrow + 1][64];
@@ -398,17 +403,18 @@ static bool vec4(const float *p, int ld) { return (ld & 3) == 0 && ((uintptr_t)p
 static void launch_layer(const float *X, int B, int K, int N, const float *W, const float *b,
                          float *Y, int act, cudaStream_t st) {
   if (N <= kNarrow) {
-    mlp_forward_narrow_kernel<<<(B + 7) / 8, 256, 0, st>>>(B, N, K, X, W, b, Y, act);
+    launch_dependent(mlp_forward_narrow_kernel, (B + 7) / 8, 256, 0, st, B, N, K, X, W, b, Y, act);
     return;
   }
   dim3 grid((N + TN - 1) / TN, (B + TM - 1) / TM);
-  mlp_gemm_kernel<MLP_FORWARD><<<grid, 256, 0, st>>>(B, N, K, X, W, b, Y, act, 0, vec4(X, K),
-                                                     vec4(W, K), vec4(Y, N));
+  launch_dependent(mlp_gemm_kernel<MLP_FORWARD>, grid, 256, 0, st, B, N, K, X, W, b, Y, act, 0,
+                   vec4(X, K), vec4(W, K), vec4(Y, N));
 }
 
 // g[i] = sum over the splits z (in order) of P[z][i]
 __global__ void grad_sum_kernel(int nsplit, int n, const float *__restrict__ P,
                                 float *__restrict__ g) {
+  dependent_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.f;
@@ -421,6 +427,7 @@ __global__ void grad_sum_kernel(int nsplit, int n, const float *__restrict__ P,
 __global__ void loss_grad_kernel(int n, const float *__restrict__ Y, const float *__restrict__ T,
                                  const float *__restrict__ mask, float inv_msum,
                                  float *__restrict__ dY, float *__restrict__ part) {
+  dependent_begin();
   __shared__ float sh[256];
   float s = 0.f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -440,6 +447,7 @@ __global__ void loss_grad_kernel(int n, const float *__restrict__ Y, const float
 __global__ void adam_kernel(int n, float *__restrict__ w, const float *__restrict__ g,
                             float *__restrict__ m, float *__restrict__ v, float lr, float b1,
                             float b2, float eps, float c1, float c2) {
+  dependent_begin();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -455,6 +463,7 @@ __global__ void gather_rows_kernel(int B, int ni, int no, const int *__restrict_
                                    const float *__restrict__ X, const float *__restrict__ T,
                                    const float *__restrict__ K, float *__restrict__ Xb,
                                    float *__restrict__ Tb, float *__restrict__ Kb) {
+  dependent_begin();
   const int64_t w = ni + 2 * no;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < B * w;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -551,7 +560,8 @@ struct Mlp {
   int backward(const float *X, const float *T, const float *Mk, int B, float msum, float *loss) {
     const int nl = layers(), no = width.back();
     const int nb = 64;
-    loss_grad_kernel<<<nb, 256, 0, st>>>(B * no, act[nl - 1], T, Mk, 1.f / msum, d_dA, d_part);
+    launch_dependent(loss_grad_kernel, nb, 256, 0, st, B * no, act[nl - 1], T, Mk, 1.f / msum,
+                     d_dA, d_part);
     float *dcur = d_dA, *dnext = d_dB;
     for (int l = nl - 1; l >= 0; l--) {
       const int K = width[l], N = width[l + 1];
@@ -565,27 +575,29 @@ struct Mlp {
       if (K <= kNarrow || N <= kNarrow) {
         const int wide_is_d = K <= kNarrow;
         dim3 g1(((wide_is_d ? N : K) + 63) / 64, nsplit);
-        mlp_grad_narrow_kernel<<<g1, 256, 0, st>>>(B, N, K, dcur, Hin, part, mchunk, wide_is_d);
+        launch_dependent(mlp_grad_narrow_kernel, g1, 256, 0, st, B, N, K, dcur, Hin, part, mchunk,
+                         wide_is_d);
       } else {
         dim3 g1((K + TN - 1) / TN, (N + TM - 1) / TM, nsplit);
-        mlp_gemm_kernel<MLP_GRAD><<<g1, 256, 0, st>>>(N, K, B, dcur, Hin, nullptr, part, 0,
-                                                      mchunk, vec4(dcur, N), vec4(Hin, K),
-                                                      vec4(part, K) && (nsplit == 1 || (N & 3) == 0));
+        launch_dependent(mlp_gemm_kernel<MLP_GRAD>, g1, 256, 0, st, N, K, B, dcur, Hin, nullptr,
+                         part, 0, mchunk, vec4(dcur, N), vec4(Hin, K),
+                         vec4(part, K) && (nsplit == 1 || (N & 3) == 0));
       }
       if (nsplit > 1)
-        grad_sum_kernel<<<(N * K + N + 255) / 256, 256, 0, st>>>(nsplit, N * K + N, d_split,
-                                                                 d_g + woff[l]);
+        launch_dependent(grad_sum_kernel, (N * K + N + 255) / 256, 256, 0, st, nsplit, N * K + N,
+                         d_split, d_g + woff[l]);
       if (l == 0) break;
       // dZ_{l-1} = (dZ W_l) (1 - H^2)  [B][K]
       const float *W = d_w + woff[l];
       if (N <= kNarrow) {
         dim3 g2((K + 255) / 256, std::min(B, 1216));
-        mlp_back_narrow_kernel<<<g2, 256, 0, st>>>(B, N, K, dcur, W, act[l - 1], dnext);
+        launch_dependent(mlp_back_narrow_kernel, g2, 256, 0, st, B, N, K, dcur, W, act[l - 1],
+                         dnext);
       } else {
         dim3 g2((K + TN - 1) / TN, (B + TM - 1) / TM);
-        mlp_gemm_kernel<MLP_BACK><<<g2, 256, 0, st>>>(B, K, N, dcur, W, act[l - 1], dnext, 0, 0,
-                                                      vec4(dcur, N), vec4(W, K),
-                                                      vec4(dnext, K) && vec4(act[l - 1], K));
+        launch_dependent(mlp_gemm_kernel<MLP_BACK>, g2, 256, 0, st, B, K, N, dcur, W, act[l - 1],
+                         dnext, 0, 0, vec4(dcur, N), vec4(W, K),
+                         vec4(dnext, K) && vec4(act[l - 1], K));
       }
       float *t = dcur;
       dcur = dnext;
@@ -603,7 +615,8 @@ struct Mlp {
   void adam(float lr, float b1, float b2, float eps) {
     adam_t++;
     const float c1 = 1.f - powf(b1, (float)adam_t), c2 = 1.f - powf(b2, (float)adam_t);
-    adam_kernel<<<304, 256, 0, st>>>(nparam, d_w, d_g, d_m, d_v, lr, b1, b2, eps, c1, c2);
+    launch_dependent(adam_kernel, 304, 256, 0, st, nparam, d_w, d_g, d_m, d_v, lr, b1, b2, eps, c1,
+                     c2);
   }
 };
 
@@ -761,8 +774,8 @@ int gb_mlp_train_device(gb_mlp *m, const float *d_x, const float *d_t, const flo
     if (ms <= 0.0) continue;
     e = cudaMemcpyAsync(M.d_idx, idx.data(), sizeof(int) * B, cudaMemcpyHostToDevice, M.st);
     if (e != cudaSuccess) return gb::cuda_fail(e, "batch");
-    gb::gather_rows_kernel<<<304, 256, 0, M.st>>>(B, ni, no, M.d_idx, d_x, d_t, d_mask, M.d_xb,
-                                                  M.d_tb, M.d_mb);
+    gb::launch_dependent(gb::gather_rows_kernel, 304, 256, 0, M.st, B, ni, no, M.d_idx, d_x, d_t,
+                         d_mask, M.d_xb, M.d_tb, M.d_mb);
     M.forward(M.d_xb, B);
     // the loss is read back on the last step only: no per-step host wait
     if (M.backward(M.d_xb, M.d_tb, M.d_mb, B, (float)ms, s + 1 == steps ? &loss : nullptr))

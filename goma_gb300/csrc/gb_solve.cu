@@ -25,6 +25,7 @@
 
 #include "gb_context.h"
 #include "gb_factor.h"
+#include "gb_launch.cuh"
 #include "gb_publish.cuh"
 #include "gb_solve.h"
 
@@ -193,6 +194,7 @@ template <class T, int OP>
 __global__ void __launch_bounds__(256, 4)
     gs_kernel(int N, int k, const T *__restrict__ V, int64_t ld, const double *__restrict__ h,
               T *__restrict__ w, double *__restrict__ part) {
+  dependent_begin();
   using A = acc_t<T>;
   constexpr int RPT = kGsRows / 32;
   __shared__ A sub[8][kGsRows];
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(256, 4)
 __global__ void __launch_bounds__(128)
     multidot_final_kernel(int nblocks, const double *__restrict__ part, double *__restrict__ out,
                           double *__restrict__ host) {
+  dependent_begin();
   __shared__ double red[4];
   const int j = blockIdx.x;
   double s = 0.0;
@@ -323,6 +326,7 @@ struct SweepIo {
 template <class T, class T2>
 __global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *__restrict__ part,
                                   double *norm, double *host, T *y, SweepIo<T2> io) {
+  dependent_begin();
   io.start();
   using A = acc_t<T>;
   __shared__ double red[kRedThreads / 32];
@@ -419,6 +423,7 @@ __global__ void to_f32_kernel(int64_t n, const double *__restrict__ x, float *__
 }
 
 __global__ void to_f64_kernel(int64_t n, const float *__restrict__ x, double *__restrict__ y) {
+  dependent_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (double)x[i];
@@ -459,6 +464,7 @@ __global__ void __launch_bounds__(256)
     spmv_kernel(int ng, const int2 *__restrict__ groups, const int64_t *__restrict__ rowptr,
                 const int *__restrict__ colidx, const T *__restrict__ vals,
                 const T *__restrict__ x, T *__restrict__ y) {
+  dependent_begin();
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPR, l = threadIdx.x % LPR;
   using A = acc_t<T>;
   A s[4] = {};
@@ -994,9 +1000,9 @@ static cudaError_t spmv(const Context *C, int lpr, const T *vals, const T *x, T 
               : 8;
   const int blocks = (int)(((int64_t)ng * lpr + threads - 1) / threads);
   switch (lpr) {
-  case 32: spmv_kernel<T, 32><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
-  case 16: spmv_kernel<T, 16><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
-  default: spmv_kernel<T, 8><<<blocks, threads, 0, st>>>(ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y);
+  case 32: launch_dependent(spmv_kernel<T, 32>, blocks, threads, 0, st, ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
+  case 16: launch_dependent(spmv_kernel<T, 16>, blocks, threads, 0, st, ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y); break;
+  default: launch_dependent(spmv_kernel<T, 8>, blocks, threads, 0, st, ng, S.d_rowgrp, C->d_rowptr, C->d_colidx, vals, x, y);
   }
   return cudaGetLastError();
 }
@@ -1281,11 +1287,11 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
   auto basis_vector = [&](const T *src, int nparts, const double *part, double *nrm, T *v) {
     double *hn = hh + (nrm - dh);
     if (flexible)
-      scale_copy_kernel<T, float><<<kRedBlocks, kRedThreads, 0, st>>>(
-          N, src, nparts, part, nrm, hn, v, sweep_io(S, S.d_t32, true));
+      launch_dependent(scale_copy_kernel<T, float>, kRedBlocks, kRedThreads, 0, st, N, src, nparts,
+                       part, nrm, hn, v, sweep_io(S, S.d_t32, true));
     else
-      scale_copy_kernel<T, T><<<kRedBlocks, kRedThreads, 0, st>>>(N, src, nparts, part, nrm, hn, v,
-                                                                  sweep_io(S, t, false));
+      launch_dependent(scale_copy_kernel<T, T>, kRedBlocks, kRedThreads, 0, st, N, src, nparts,
+                       part, nrm, hn, v, sweep_io(S, t, false));
   };
   GB_CU(cudaMemsetAsync(x, 0, sizeof(T) * N, st), "x0");
   double bnorm;
@@ -1314,7 +1320,8 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
           if (direct ? sync_free_apply<float>(&S, (float *)S.d_sweep_y + N, S.d_t32, st)
                      : S.apply_prec32(st))
             return -1;
-          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
+          launch_dependent(to_f64_kernel, kRedBlocks, kRedThreads, 0, st, N, S.d_t32,
+                           S.d_Z + k * ld);
           z = S.d_Z + k * ld;
         }
       }
@@ -1339,11 +1346,15 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
       // CGS2 on the device; the host reads both passes and the norm in hh
       std::vector<double> hcol(j + 2, 0.0);
       double *dh1 = dh, *dh2 = dh + (m + 2), *dnrm = dh + 2 * (m + 2);
-      gs_kernel<T, GS_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, nullptr, w, dpart);
-      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh1, hh);
-      gs_kernel<T, GS_SUB_DOTS><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh1, w, dpart);
-      multidot_final_kernel<<<j + 1, 128, 0, st>>>(gs_blocks, dpart, dh2, hh + (m + 2));
-      gs_kernel<T, GS_SUB_NORM><<<gs_blocks, 256, 0, st>>>(N, j + 1, V, ld, dh2, w, dpart);
+      launch_dependent(gs_kernel<T, GS_DOTS>, gs_blocks, 256, 0, st, N, j + 1, V, ld, nullptr, w,
+                       dpart);
+      launch_dependent(multidot_final_kernel, j + 1, 128, 0, st, gs_blocks, dpart, dh1, hh);
+      launch_dependent(gs_kernel<T, GS_SUB_DOTS>, gs_blocks, 256, 0, st, N, j + 1, V, ld, dh1, w,
+                       dpart);
+      launch_dependent(multidot_final_kernel, j + 1, 128, 0, st, gs_blocks, dpart, dh2,
+                       hh + (m + 2));
+      launch_dependent(gs_kernel<T, GS_SUB_NORM>, gs_blocks, 256, 0, st, N, j + 1, V, ld, dh2, w,
+                       dpart);
       basis_vector(w, gs_blocks, dpart, dnrm, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "Arnoldi step");
       GB_CU(cudaEventRecord(S.ev_h, st), "h");
@@ -1428,6 +1439,7 @@ __global__ void __launch_bounds__(256, 2)
                   T *__restrict__ w, const int *__restrict__ tseg,
                   const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
                   double *__restrict__ part) {
+  dependent_begin();
   using A = acc_t<T>;
   __shared__ double red[8][32];
   __shared__ double cs[32];
@@ -1491,6 +1503,7 @@ __global__ void __launch_bounds__(256, 2)
 __global__ void seg_reduce_kernel(int nseg, int k, const int *__restrict__ tptr,
                                   const double *__restrict__ part, double *__restrict__ out,
                                   double *__restrict__ host) {
+  dependent_begin();
   const int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= nseg * k) return;
   const int sg = u / k, j = u - sg * k;
@@ -1526,6 +1539,7 @@ __global__ void seg_scale_kernel(const T *src, const double *__restrict__ norm2,
                                  const int *__restrict__ active, const int *__restrict__ tseg,
                                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
                                  T *dst, SweepIo<T2> io) {
+  dependent_begin();
   io.start();
   const int t = blockIdx.x, sg = tseg[t];
   __shared__ double inv;
@@ -1559,26 +1573,24 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
   double *o1 = S.d_segout, *o2 = o1 + 32 * ns, *o3 = o2 + 32 * ns;
   double *h1 = S.h_segout, *h2 = h1 + 32 * ns, *h3 = h2 + 32 * ns;
   auto reduce = [&](int k, double *out) {
-    seg_reduce_kernel<<<(ns * k + 7) / 8, 256, 0, st>>>(ns, k, S.d_tile_ptr, S.d_segpart, out,
-                                                        h1 + (out - o1));
+    launch_dependent(seg_reduce_kernel, (ns * k + 7) / 8, 256, 0, st, ns, k, S.d_tile_ptr,
+                     S.d_segpart, out, h1 + (out - o1));
   };
   // w . v on every block
   auto dot1 = [&](const T *v, T *wv, double *out) {
-    seg_gs_kernel<T, GS_DOTS><<<nt, 256, 0, st>>>(1, v, ld, nullptr, wv, S.d_tile_seg,
-                                                  S.d_tile_beg, S.d_tile_end, S.d_segpart);
+    launch_dependent(seg_gs_kernel<T, GS_DOTS>, nt, 256, 0, st, 1, v, ld, nullptr, wv, S.d_tile_seg,
+                     S.d_tile_beg, S.d_tile_end, S.d_segpart);
     reduce(1, out);
   };
   if (S.direct_sweeps() && S.ensure_sweep_y()) return -1;
   // v = src / norm per block, and what the preconditioner wants of it
   auto basis_vector = [&](const T *src, T *v) {
     if (flexible)
-      seg_scale_kernel<T, float><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
-                                                     S.d_tile_beg, S.d_tile_end, v,
-                                                     sweep_io(S, S.d_t32, true));
+      launch_dependent(seg_scale_kernel<T, float>, nt, 256, 0, st, src, o3, S.d_segactive,
+                       S.d_tile_seg, S.d_tile_beg, S.d_tile_end, v, sweep_io(S, S.d_t32, true));
     else
-      seg_scale_kernel<T, T><<<nt, 256, 0, st>>>(src, o3, S.d_segactive, S.d_tile_seg,
-                                                 S.d_tile_beg, S.d_tile_end, v,
-                                                 sweep_io(S, t, false));
+      launch_dependent(seg_scale_kernel<T, T>, nt, 256, 0, st, src, o3, S.d_segactive, S.d_tile_seg,
+                       S.d_tile_beg, S.d_tile_end, v, sweep_io(S, t, false));
   };
   std::vector<int> active(ns, 1), done(ns, 0);
   std::vector<double> bnorm(ns), beta(ns), coef(32 * (size_t)ns);
@@ -1625,7 +1637,8 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
           if (direct ? sync_free_apply<float>(&S, (float *)S.d_sweep_y + N, S.d_t32, st)
                      : S.apply_prec32(st))
             return -1;
-          to_f64_kernel<<<kRedBlocks, kRedThreads, 0, st>>>(N, S.d_t32, S.d_Z + k * ld);
+          launch_dependent(to_f64_kernel, kRedBlocks, kRedThreads, 0, st, N, S.d_t32,
+                           S.d_Z + k * ld);
           z = S.d_Z + k * ld;
         }
       }
@@ -1642,14 +1655,14 @@ static int gmres_seg(Context *C, const T *b, T *x, double tol, int maxit, int m,
     double before = HUGE_VAL;
     for (; j < m && total < maxit; j++) {
       if (!ahead && apply_operator(j)) return -1;
-      seg_gs_kernel<T, GS_DOTS><<<nt, 256, 0, st>>>(j + 1, V, ld, nullptr, w, S.d_tile_seg,
-                                                    S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      launch_dependent(seg_gs_kernel<T, GS_DOTS>, nt, 256, 0, st, j + 1, V, ld, nullptr, w,
+                       S.d_tile_seg, S.d_tile_beg, S.d_tile_end, S.d_segpart);
       reduce(j + 1, o1);
-      seg_gs_kernel<T, GS_SUB_DOTS><<<nt, 256, 0, st>>>(j + 1, V, ld, o1, w, S.d_tile_seg,
-                                                        S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      launch_dependent(seg_gs_kernel<T, GS_SUB_DOTS>, nt, 256, 0, st, j + 1, V, ld, o1, w,
+                       S.d_tile_seg, S.d_tile_beg, S.d_tile_end, S.d_segpart);
       reduce(j + 1, o2);
-      seg_gs_kernel<T, GS_SUB_NORM><<<nt, 256, 0, st>>>(j + 1, V, ld, o2, w, S.d_tile_seg,
-                                                        S.d_tile_beg, S.d_tile_end, S.d_segpart);
+      launch_dependent(seg_gs_kernel<T, GS_SUB_NORM>, nt, 256, 0, st, j + 1, V, ld, o2, w,
+                       S.d_tile_seg, S.d_tile_beg, S.d_tile_end, S.d_segpart);
       reduce(1, o3);
       basis_vector(w, V + (j + 1) * ld);
       GB_CU(cudaGetLastError(), "batched Arnoldi step");

@@ -58,6 +58,7 @@
 #include <vector>
 
 #include "gb_context.h"
+#include "gb_launch.cuh"
 #include "gb_publish.cuh"
 #include "gb_sweep.h"
 
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(NT, MINB)
   for (int k = threadIdx.x; k < kRing * kMaxDofs; k += NT) set_unpublished(&ring[0][0] + k);
   if (threadIdx.x < kRing) drawn[threadIdx.x] = -1;
   if (threadIdx.x == 0) claimed = -1;
+  dependent_begin();
   __syncthreads();
   const int limit = (int)min(g.spin_limit, 0x7fffffffLL);
   bool gave_up = false;
@@ -357,7 +359,7 @@ template <class T, bool WIDE, int NT, int MINB>
 static cudaError_t launch_lines(const LineArgs &a, const T *vals, const T *b, T *x, int sms,
                                 bool one_cta, cudaStream_t st) {
   const int grid = one_cta ? 1 : std::min(a.nlines, MINB * sms);
-  line_sweep_kernel<T, WIDE, NT, MINB><<<grid, NT, 0, st>>>(a, vals, b, x);
+  launch_dependent(line_sweep_kernel<T, WIDE, NT, MINB>, grid, NT, 0, st, a, vals, b, x);
   return cudaGetLastError();
 }
 
