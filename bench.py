@@ -269,20 +269,21 @@ def element_flops(path):
     Jacobian) of the element kernel of `path`, counted from its algorithm.
 
     Path 4 (sum factorisation, the automatic path): isoparametric passes
-    7 fields x (2 + 3 + 4) x 27 outputs x 5; per-point set-up ~263 x 27;
-    gradient tables 729 x 18; sum-factorisation stages 16 x (81 + 243) x 5;
-    residual rows 108 x 27 x 8; J_mP 324 x 27 x 2; upper triangle of the
-    81 x 81 gradient product 3,321 x 27 x 2; node pairs 729 x 113.
+    7 fields x (2 + 3 + 4) x 27 outputs x 5; per-point set-up ~330 x 27;
+    gradient tables 729 x 18; the contractions of 13 mass matrices (54, 108,
+    216 values a stage) and 3 advection terms (54 or 81, 108 or 162, 324) x 5;
+    four residual rows 27 x 48; J_mP 324 x 27 x 2; the gradient products of
+    378 node pairs, 9 x 27 x 2 each; their blocks 378 x 12 + 729 x 25.
     Paths 1-3 do the dense quadrature-point contractions: 2 Q n_loc^2 (d+1)."""
     if path in (0, 4):
         iso = 7 * (2 + 3 + 4) * 27 * 5
-        qp = 263 * 27
+        qp = 330 * 27
         tables = 729 * 18
-        stages = 16 * (81 + 243) * 5
-        resid = 108 * 27 * 8
+        stages = ((15 * 54 + 81) + (14 * 108 + 2 * 162) + (13 * 216 + 3 * 324)) * 5
+        resid = 4 * 27 * 48
         jmp = 324 * 27 * 2
-        h = 3321 * (27 * 2 + 2)
-        pairs = 729 * 113
+        h = 378 * 9 * 27 * 2
+        pairs = 378 * 12 + 729 * 25
         return float(iso + qp + tables + stages + resid + jmp + h + pairs)
     nloc = 4 * 27 + 4
     return 2.0 * 27 * nloc * nloc * 4

@@ -20,6 +20,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <future>
+#include <system_error>
 #include <type_traits>
 #include <vector>
 
@@ -876,17 +878,24 @@ int Solver::init(Context *c, int krylov) {
           "block inverse offsets");
     GB_CU(cudaMalloc(&d_binv, sizeof(double) * inv_len), "block inverses");
   }
+  // the two sweeps' tables and the schedule, side by side
   IluSchedule S;
-  build_ilu_schedule(*LP, S);
+  {
+    LineTables lo, hi;
+    std::future<int> up;
+    try {
+      up = std::async(std::launch::async, [&] { return build_line_tables(*LP, true, hi); });
+    } catch (const std::system_error &) {  // no thread to be had
+    }
+    int bad = build_line_tables(*LP, false, lo);
+    build_ilu_schedule(*LP, S);
+    bad |= up.valid() ? up.get() : build_line_tables(*LP, true, hi);
+    if (bad) return fail("a matrix row is too long for the sweeps");
+    if (line_lo.upload(lo) || line_up.upload(hi)) return -1;
+  }
   lo_ptr = S.lo_ptr;
   up_ptr = S.up_ptr;
   num_levels = (int)lo_ptr.size() - 1;
-  {
-    LineTables lo, hi;
-    if (build_line_tables(*LP, false, lo) || build_line_tables(*LP, true, hi))
-      return fail("a matrix row is too long for the sweeps");
-    if (line_lo.upload(lo) || line_up.upload(hi)) return -1;
-  }
   GB_CU(cudaMalloc(&d_lo_nodes, sizeof(int) * S.lo_nodes.size()), "sched");
   GB_CU(cudaMemcpy(d_lo_nodes, S.lo_nodes.data(), sizeof(int) * S.lo_nodes.size(),
                    cudaMemcpyHostToDevice), "sched");
