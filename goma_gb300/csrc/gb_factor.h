@@ -20,6 +20,7 @@ struct IluArgs {
   int maxnb, lmax, blkmax, maxnr;  // neighbours, row length, block-row values, unknowns
   double tau;           // pivot floor
   int *nfix;            // floored pivots
+  void *rpiv;           // reciprocal pivots, [unknowns] of the factors' type
   int *done;            // [num_nodes] set when a node's rows are final, then the ticket
   int *error;           // set when a wait gave up
   long long spin_limit; // polls before a wait gives up

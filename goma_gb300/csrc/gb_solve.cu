@@ -753,6 +753,7 @@ static IluArgs ilu_args(const Solver *S, const Context *C, int *nfix) {
   g.maxnr = L.nvn + L.npres;
   g.tau = S->pivot_tau;
   g.nfix = nfix;
+  g.rpiv = S->d_rpiv;
   g.done = S->d_done;
   g.error = (int *)(S->d_flags + 4);
   g.spin_limit = kSpinLimit;
@@ -932,6 +933,8 @@ int Solver::init(Context *c, int krylov) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  GB_CU(cudaMalloc(&d_rpiv, sizeof(double) * N), "reciprocal pivots");
+  owned.push_back(d_rpiv);
   GB_CU(cudaMalloc(&d_lu, sizeof(double) * nnz), "ILU factors");
   GB_CU(cudaMalloc(&d_scale, sizeof(double) * N), "scale");
   const size_t wk = (size_t)(kRedBlocks * 3 + (krylov + 2) * kGsBlocks + 4 * (krylov + 2) + 96);

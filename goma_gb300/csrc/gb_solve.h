@@ -85,6 +85,7 @@ struct Solver {
   // largest node neighbourhood, row length and block row (values)
   int maxnb = 0, lmax = 0, blkmax = 0;
   int *d_done = nullptr;        // nodes whose factors are final (and the next node to draw)
+  void *d_rpiv = nullptr;       // reciprocal pivots of the factorisation
   double *d_scale = nullptr;
   double *d_work = nullptr;     // reduction scratch
   double *h_work = nullptr;     // pinned host mirror
