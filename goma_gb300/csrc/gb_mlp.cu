@@ -458,6 +458,44 @@ __global__ void adam_kernel(int n, float *__restrict__ w, const float *__restric
   }
 }
 
+// All layers' gradients from their splits and, with adam, the parameters'
+// step: one launch for the whole network instead of a sum a layer and Adam (a
+// training step of 8-256-256-256-1: 18 -> 14 launches, 14 -> 5 us of sums and
+// step).
+constexpr int kMaxFused = 16;  // layers
+struct LayerTab {
+  int n = 0, off[kMaxFused] = {}, len[kMaxFused] = {};  // in the parameters
+};
+struct AdamArgs {
+  float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(256)
+    grad_step_kernel(int n, LayerTab L, int nsplit, const float *P, float *g, bool adam,
+                     float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
+                     AdamArgs a) {
+  dependent_begin();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int off = 0, len = 0;
+#pragma unroll
+  for (int l = 0; l < kMaxFused; l++)
+    if (l < L.n && i >= L.off[l]) {
+      off = L.off[l];
+      len = L.len[l];
+    }
+  const float *p = P + (int64_t)off * nsplit + (i - off);
+  float s = 0.f;
+#pragma unroll 8
+  for (int z = 0; z < nsplit; z++) s += p[(int64_t)z * len];
+  g[i] = s;
+  if (!adam) return;
+  const float mi = a.b1 * m[i] + (1.f - a.b1) * s;
+  const float vi = a.b2 * v[i] + (1.f - a.b2) * s * s;
+  m[i] = mi;
+  v[i] = vi;
+  w[i] -= a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+}
+
 // rows idx[b] of X[n][ni], T[n][no] and K[n][no] -> Xb, Tb, Kb
 __global__ void gather_rows_kernel(int B, int ni, int no, const int *__restrict__ idx,
                                    const float *__restrict__ X, const float *__restrict__ T,
@@ -520,6 +558,8 @@ struct Mlp {
     return m;
   }
   int layers() const { return (int)width.size() - 1; }
+  // the splits of all layers at once: small networks
+  bool fused() const { return layers() <= kMaxFused && nparam <= (2 << 20); }
   int ensure(int B) {
     if (B <= cap) return 0;
     for (float *a : act) cudaFree(a);
@@ -542,7 +582,9 @@ struct Mlp {
         cudaMalloc(&d_idx, sizeof(int) * (size_t)B) != cudaSuccess)
       return fail("MLP scratch");
     if (!d_split &&
-        cudaMalloc(&d_split, sizeof(float) * (size_t)kMaxSplit * maxw() * (maxw() + 1)) != cudaSuccess)
+        cudaMalloc(&d_split, sizeof(float) * kMaxSplit *
+                                 (fused() ? (size_t)nparam : (size_t)maxw() * (maxw() + 1))) !=
+            cudaSuccess)
       return fail("MLP scratch");
     cap = B;
     return 0;
@@ -557,21 +599,25 @@ struct Mlp {
   }
   // gradient of sum mask (Y - T)^2 / sum(mask) into d_g; with loss != NULL
   // also waits for and returns the loss (host)
-  int backward(const float *X, const float *T, const float *Mk, int B, float msum, float *loss) {
+  // and with adam takes the step
+  int backward(const float *X, const float *T, const float *Mk, int B, float msum, float *loss,
+               const AdamArgs *adam = nullptr) {
     const int nl = layers(), no = width.back();
     const int nb = 64;
     launch_dependent(loss_grad_kernel, nb, 256, 0, st, B * no, act[nl - 1], T, Mk, 1.f / msum,
                      d_dA, d_part);
     float *dcur = d_dA, *dnext = d_dB;
+    const int nsplit = std::max(1, std::min(kMaxSplit, B / 128));
+    const int mchunk = ((B + nsplit - 1) / nsplit + TK - 1) / TK * TK;
+    LayerTab tab;
     for (int l = nl - 1; l >= 0; l--) {
       const int K = width[l], N = width[l + 1];
       const float *Hin = l == 0 ? X : act[l - 1];
       // dW_l = dZ^T Hin  [N][K] and db_l = colsum dZ, which follows it in
       // d_g; the batch split over up to kMaxSplit CTA layers so that the grid
       // covers the GPU
-      const int nsplit = std::max(1, std::min(kMaxSplit, B / 128));
-      const int mchunk = ((B + nsplit - 1) / nsplit + TK - 1) / TK * TK;
-      float *part = nsplit == 1 ? d_g + woff[l] : d_split;
+      float *part = nsplit == 1 ? d_g + woff[l]
+                                : d_split + (fused() ? (size_t)woff[l] * nsplit : 0);
       if (K <= kNarrow || N <= kNarrow) {
         const int wide_is_d = K <= kNarrow;
         dim3 g1(((wide_is_d ? N : K) + 63) / 64, nsplit);
@@ -583,7 +629,7 @@ struct Mlp {
                          part, 0, mchunk, vec4(dcur, N), vec4(Hin, K),
                          vec4(part, K) && (nsplit == 1 || (N & 3) == 0));
       }
-      if (nsplit > 1)
+      if (nsplit > 1 && !fused())
         launch_dependent(grad_sum_kernel, (N * K + N + 255) / 256, 256, 0, st, nsplit, N * K + N,
                          d_split, d_g + woff[l]);
       if (l == 0) break;
@@ -603,6 +649,18 @@ struct Mlp {
       dcur = dnext;
       dnext = t;
     }
+    if (fused() && (nsplit > 1 || adam)) {
+      tab.n = nl;
+      for (int l = 0; l < nl; l++) {
+        tab.off[l] = woff[l];
+        tab.len[l] = width[l + 1] * (width[l] + 1);
+      }
+      launch_dependent(grad_step_kernel, (nparam + 255) / 256, 256, 0, st, nparam, tab, nsplit,
+                       nsplit == 1 ? d_g : d_split, d_g, adam != nullptr, d_w, d_m, d_v,
+                       adam ? *adam : AdamArgs{});
+    } else if (adam) {
+      launch_adam(*adam);
+    }
     if (!loss) return 0;  // no loss wanted: nothing to wait for
     cudaMemcpyAsync(h_part, d_part, sizeof(float) * nb, cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
@@ -612,11 +670,13 @@ struct Mlp {
     if (loss) *loss = (float)(s / msum);
     return 0;
   }
-  void adam(float lr, float b1, float b2, float eps) {
+  AdamArgs adam_args(float lr, float b1, float b2, float eps) {
     adam_t++;
-    const float c1 = 1.f - powf(b1, (float)adam_t), c2 = 1.f - powf(b2, (float)adam_t);
-    launch_dependent(adam_kernel, 304, 256, 0, st, nparam, d_w, d_g, d_m, d_v, lr, b1, b2, eps, c1,
-                     c2);
+    return {lr, b1, b2, eps, 1.f - powf(b1, (float)adam_t), 1.f - powf(b2, (float)adam_t)};
+  }
+  void launch_adam(const AdamArgs &a) {
+    launch_dependent(adam_kernel, 304, 256, 0, st, nparam, d_w, d_g, d_m, d_v, a.lr, a.b1, a.b2,
+                     a.eps, a.c1, a.c2);
   }
 };
 
@@ -739,7 +799,7 @@ int gb_mlp_loss_grad_device(gb_mlp *m, const float *d_x, const float *d_t, const
 
 int gb_mlp_adam_step(gb_mlp *m, float lr, float beta1, float beta2, float eps) {
   if (!m) return gb::fail("NULL argument");
-  m->m.adam(lr, beta1, beta2, eps);
+  m->m.launch_adam(m->m.adam_args(lr, beta1, beta2, eps));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : gb::cuda_fail(e, "Adam");
 }
@@ -778,9 +838,9 @@ int gb_mlp_train_device(gb_mlp *m, const float *d_x, const float *d_t, const flo
                          d_mask, M.d_xb, M.d_tb, M.d_mb);
     M.forward(M.d_xb, B);
     // the loss is read back on the last step only: no per-step host wait
-    if (M.backward(M.d_xb, M.d_tb, M.d_mb, B, (float)ms, s + 1 == steps ? &loss : nullptr))
+    const gb::AdamArgs step = M.adam_args(lr, 0.9f, 0.999f, 1e-8f);
+    if (M.backward(M.d_xb, M.d_tb, M.d_mb, B, (float)ms, s + 1 == steps ? &loss : nullptr, &step))
       return -1;
-    M.adam(lr, 0.9f, 0.999f, 1e-8f);
   }
   e = cudaStreamSynchronize(M.st);
   if (e != cudaSuccess) return gb::cuda_fail(e, "MLP training");

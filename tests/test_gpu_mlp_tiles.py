@@ -50,3 +50,24 @@ def test_forward_and_gradients(shape, n, shift):
     assert abs(loss - loss_ref) <= 1e-5 * loss_ref
     assert np.abs(net.grads() - g_ref).max() <= 1e-4 * np.abs(g_ref).max()
     net.close()
+
+
+@pytest.mark.parametrize("shape,n", [((8, 256, 3, 1), 4161), ((9, 72, 2, 9), 65),
+                                     ((3, 20, 18, 2), 300)])
+def test_a_training_step_is_the_gradient_and_an_adam_step(shape, n):
+    """All layers' sums and the step in one launch (up to 16 layers), against
+    the gradient's own launches and a step after them: the same operations."""
+    import torch
+    from goma_gb300.mlp import GpuMLP
+    rng = np.random.default_rng(n)
+    x, t, m = (torch.from_numpy(rng.uniform(0.1, 1, (n, k)).astype(np.float32)).cuda()
+               for k in (shape[0], shape[3], shape[3]))
+    nets = [GpuMLP(*shape, seed=4) for _ in range(2)]
+    for k in range(2):
+        nets[0].train(x, t, m, 1, batch=n, lr=1e-2)
+        nets[1].loss_grad(x, t, m)
+        nets[1].adam_step(lr=1e-2)
+        assert np.array_equal(nets[0].grads(), nets[1].grads())
+        assert np.array_equal(nets[0].params(), nets[1].params())
+    for net in nets:
+        net.close()
