@@ -148,7 +148,10 @@ struct SumF32 {
     e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z)));
     s = t;
   }
-  __device__ __forceinline__ double get() const { return (double)s + (double)e; }
+  // an infinite sum has no error to add (its two-sum is NaN)
+  __device__ __forceinline__ double get() const {
+    return e == e ? (double)s + (double)e : (double)s;
+  }
 };
 template <class T>
 struct SumOf {
