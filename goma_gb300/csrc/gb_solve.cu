@@ -882,14 +882,17 @@ int Solver::init(Context *c, int krylov) {
           "block inverse offsets");
     GB_CU(cudaMalloc(&d_binv, sizeof(double) * inv_len), "block inverses");
   }
-  // the two sweeps' tables and the schedule, side by side
+  // the two sweeps' tables and the schedule, side by side where that takes
+  // longer than starting a thread and its team (~1 ms)
   IluSchedule S;
   {
     LineTables lo, hi;
     std::future<int> up;
-    try {
-      up = std::async(std::launch::async, [&] { return build_line_tables(*LP, true, hi); });
-    } catch (const std::system_error &) {  // no thread to be had
+    if (LP->num_nodes > 8192) {
+      try {
+        up = std::async(std::launch::async, [&] { return build_line_tables(*LP, true, hi); });
+      } catch (const std::system_error &) {  // no thread to be had
+      }
     }
     int bad = build_line_tables(*LP, false, lo);
     build_ilu_schedule(*LP, S);
