@@ -584,10 +584,12 @@ static cudaError_t launch_2d(const AsmArgs &a, const S2Tables *tb, int nelem, co
                       ? launch_elems<ENERGY, CARREAU, JAC, 1, 64>(a, tb, nelem, s, st)
                       : launch_elems<ENERGY, CARREAU, JAC, 4, 128>(a, tb, nelem, s, st);
   if (e != cudaSuccess) return e;
-  const size_t sm = JAC ? sizeof(double) * 4 * (size_t)nd.blkmax : 0;
+  const size_t sm = JAC ? s2_rows_smem(nd.blkmax) : 0;
   auto k = assemble_rows_kernel<ENERGY, JAC>;
   if (JAC) {
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    // the limit belongs to the process: the same for every mesh, so that a
+    // thread with shorter rows does not lower it before this launch
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kS2RowsSmemMax);
     if (e != cudaSuccess) return e;
   }
   launch_dependent(k, (nd.num_nodes + 3) / 4, 128, sm, st, a, nd, s);

@@ -382,8 +382,8 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
 }
 
 int Context::kernel_path(bool jacobian) const {
-  // the 2-D rows are built in shared memory (four nodes a block)
-  if (L.dim != 3) return path == 1 || sizeof(double) * 4 * (size_t)L.blkmax > 200 * 1024 ? 1 : 5;
+  // the 2-D rows are built in shared memory
+  if (L.dim != 3) return path == 1 || s2_rows_smem(L.blkmax) > kS2RowsSmemMax ? 1 : 5;
   // a heat source: the scalar kernel
   if (mat.hsm != GB_HEAT_SOURCE_NONE) return 1;
   const bool gemm_ok = !carreau && mat.viscosity > 0.0;

@@ -133,6 +133,9 @@ void build_s2_tables(const double *tab_phi, const double *tab_dphi, const double
                      const double *pt, const int (*loc9)[2], const double *ell,
                      const double *dell, S2Tables &T);
 size_t s2_scratch_values(bool energy, bool jac);  // per element
+// shared memory of the row kernel (four nodes a block) and the most it takes
+inline size_t s2_rows_smem(int blkmax) { return sizeof(double) * 4 * (size_t)blkmax; }
+constexpr int kS2RowsSmemMax = 200 * 1024;
 cudaError_t launch_assemble_2d(const AsmArgs &a, bool energy, bool carreau, bool jac,
                                const S2Tables *tb, int nelem, const S2Nodes &nd, double *scratch,
                                int sms, cudaStream_t st);

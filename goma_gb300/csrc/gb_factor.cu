@@ -378,7 +378,9 @@ static cudaError_t launch_ilu(const IluArgs &g, const double *A, T *lu, int sms,
                               cudaStream_t st) {
   const size_t sm = ilu_smem_bytes(sizeof(T), g);
   auto k = ilu0_kernel<T, NT, MR>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // the limit belongs to the process: the same for every problem, so that a
+  // thread with shorter rows does not lower it before this launch
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIluSmemMax);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, sm);

@@ -26,7 +26,8 @@ struct IluArgs {
   long long spin_limit; // polls before a wait gives up
 };
 
-// Shared memory of one CTA for elements of size tsize.
+// Shared memory of one CTA for elements of size tsize, and the most there is.
+constexpr int kIluSmemMax = 227 * 1024;
 size_t ilu_smem_bytes(size_t tsize, const IluArgs &g);
 // lu = ILU(0) factors of A in its pattern; g.done cleared beforehand
 template <class T>

@@ -927,7 +927,7 @@ int Solver::init(Context *c, int krylov) {
     const size_t rows = sizeof(int64_t) * maxnb * maxnr + sizeof(double) * (maxnr * lmax + 800) +
                         sizeof(int) * (15 * (size_t)maxnb + 4);
     const IluArgs g = ilu_args(this, C, nullptr);
-    if (rows > 200 * 1024 || ilu_smem_bytes(sizeof(double), g) > 227 * 1024)
+    if (rows > 200 * 1024 || ilu_smem_bytes(sizeof(double), g) > kIluSmemMax)
       return fail("ILU(0) block row does not fit in shared memory");
   }
   GB_CU(cudaMalloc(&d_done, sizeof(int) * (size_t)(LP->num_nodes + 1)), "ILU flags");

@@ -1,0 +1,60 @@
+"""The host side of the 2-D assembly, on a CUDA runtime without a GPU
+(fake_cudart.c)."""
+import os
+
+import pytest
+
+from goma_gb300 import _lib
+from tests import fake_runtime
+
+pytestmark = pytest.mark.skipif(not os.path.exists(_lib.LIB_PATH),
+                                reason="libgbnewton.so is not built")
+
+
+MESHES = """
+    def fan(n):
+        # n quadrilaterals around node 0
+        t = np.pi * np.arange(2 * n) / n
+        rim = np.stack([np.cos(t), np.sin(t)], 1)
+        mid = 0.5 * (rim + np.roll(rim, -1, 0))
+        centroid = 0.25 * (rim[0::2] + rim[1::2] + np.roll(rim[0::2], -1, 0))
+        i = np.arange(n)
+        j, c = (i + 1) % n, 1 + 2 * i        # the next spoke; first corner on the rim
+        m = pb.box_mesh(2, 1, 1)
+        m.coords = np.concatenate([[[0.0, 0.0]], rim, mid, 0.5 * rim[0::2], centroid])
+        m.conn = np.ascontiguousarray(np.stack(
+            [0 * i, c, c + 1, 1 + 2 * j, 1 + 4 * n + i, 2 * n + c, 2 * n + c + 1, 1 + 4 * n + j,
+             1 + 5 * n + i], 1), np.int32)
+        m.node_sets = [np.array([1], np.int32) for _ in m.node_sets]
+        return m
+    big = GomaNewton(pb.lid_cavity_2d(0, mesh=fan(60)))
+    small = GomaNewton(cavity(3, 3))
+    rp, _ = big.csr_pattern()
+    assert 4 * 8 * (rp[2] - rp[0]) > 48 * 1024  # the row kernel: four nodes a block
+"""
+
+
+@pytest.mark.parametrize("call", ["fill", "solve"])
+def test_a_call_between_another_ones_launches(call, tmp_path):
+    """A kernel's limit of dynamic shared memory belongs to the process: a
+    second thread with a mesh of shorter rows, here between any attribute that
+    the first sets and its launch, leaves the first one's launches possible."""
+    fake_runtime.run(MESHES + """
+    def fill(g):
+        return g._L.gb_matrix_fill_full_device(g.h, g.d_x, g.d_R, g.d_vals, None)
+    def solve(g):
+        opts, its, rr = g.newton_opts(), ctypes.c_int(), ctypes.c_double()
+        return g._L.gb_linear_solve_device(g.h, g.d_vals, g.d_R, g.d_x, ctypes.byref(opts),
+                                           ctypes.byref(its), ctypes.byref(rr))
+    call, calls, inside = %s, [], []
+    @ctypes.CFUNCTYPE(None)
+    def other_thread():
+        if not inside:
+            inside.append(1)
+            calls.append(call(small))
+            inside.pop()
+    ctypes.c_void_p.in_dll(fake, "fake_attribute_set").value = ctypes.cast(
+        other_thread, ctypes.c_void_p).value
+    own = [call(big) for _ in range(3)]
+    assert calls and not any(calls) and not any(own), (own, calls)
+    """ % call, tmp_path)
