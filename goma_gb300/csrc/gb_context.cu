@@ -333,7 +333,8 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
     const S2Nodes nd{L.num_nodes, d_ne_ptr, d_ne_list, L.blkmax};
     e = launch_assemble_2d(a, L.energy != 0, carreau, vals != nullptr, d_s2, L.num_elems, nd,
                            blocks, num_sms, st);
-    if (e == cudaSuccess) e = cudaFreeAsync(blocks, st);
+    const cudaError_t f = cudaFreeAsync(blocks, st);  // also after a failed launch
+    if (e == cudaSuccess) e = f;
     if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
   } else {
     e = cudaMemsetAsync(R, 0, sizeof(double) * L.N, st);

@@ -58,3 +58,18 @@ def test_a_call_between_another_ones_launches(call, tmp_path):
     own = [call(big) for _ in range(3)]
     assert calls and not any(calls) and not any(own), (own, calls)
     """ % call, tmp_path)
+
+
+def test_a_failed_launch_gives_the_element_blocks_back(tmp_path):
+    """Whichever of the two launches fails, the call returns an error and holds
+    no memory; the next call works."""
+    fake_runtime.run("""
+    gn = GomaNewton(cavity(5, 4))
+    fill = lambda: gn._L.gb_matrix_fill_full_device(gn.h, gn.d_x, gn.d_R, gn.d_vals, None)
+    live, fail = ll("fake_pool_live"), integer("fake_fail_launch")
+    for nth in (0, 1):
+        fail.value = nth
+        assert fill() == -1
+        assert live.value == 0
+        assert fill() == 0 and live.value == 0
+    """, tmp_path)
