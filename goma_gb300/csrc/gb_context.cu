@@ -275,7 +275,7 @@ int Context::init(const gb_problem_desc *d) {
   if ((e = cudaMalloc(&d_R, sizeof(double) * L.N)) != cudaSuccess) return cuda_fail(e, "R");
   if ((e = cudaMalloc(&d_vals, sizeof(double) * L.nnz)) != cudaSuccess)
     return cuda_fail(e, "CSR values");
-  if ((e = cudaMalloc(&d_status, sizeof(int) * 2)) != cudaSuccess) return cuda_fail(e, "status");
+  if ((e = cudaMalloc(&d_status, sizeof(int) * 4)) != cudaSuccess) return cuda_fail(e, "status");
   return reset_status();
 }
 
@@ -313,35 +313,58 @@ AsmArgs Context::args(const double *x, double *R, double *vals) const {
   return a;
 }
 
+// Flow rows of a 2-D mesh from element blocks (every entry of R and, with it,
+// vals).  cudaErrorMemoryAllocation: no room for the blocks, nothing done.
+cudaError_t Context::assemble_blocks(const AsmArgs &a, bool jac, cudaStream_t st) {
+  const size_t bytes =
+      sizeof(double) * s2_scratch_values(L.energy != 0, jac) * (size_t)L.num_elems;
+  double *blocks = nullptr;
+  if (cudaMallocFromPoolAsync((void **)&blocks, bytes, pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaErrorMemoryAllocation;
+  }
+  const S2Nodes nd{L.num_nodes, d_ne_ptr, d_ne_list, L.blkmax};
+  const cudaError_t e = launch_assemble_2d(a, L.energy != 0, carreau, jac, d_s2, L.num_elems, nd,
+                                           blocks, num_sms, st);
+  const cudaError_t f = cudaFreeAsync(blocks, st);  // also after a failed launch
+  kernel_launches += timing ? 2 : 0;
+  return e != cudaSuccess ? e : f;
+}
+
 int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st) {
   if (!st) st = stream;
   cudaError_t e;
   AsmArgs a = args(x, R, vals);
   const int ncol = (int)L.color_ptr.size() - 1;
   int kp = kernel_path(vals != nullptr);
-  double *blocks = nullptr;  // element blocks of the 2-D path
+  if (timing) cudaEventRecord(ev_k0, st);
+  // Where there is no room for the Jacobian's blocks the scalar kernel takes
+  // over; R then comes from the residual's blocks (a nineteenth of the size)
+  // all the same, as a residual-only assembly beside it forms it.
+  bool scalar_jac = false;
   if (kp == 5) {
-    const size_t bytes = sizeof(double) * s2_scratch_values(L.energy != 0, vals != nullptr) *
-                         (size_t)L.num_elems;
-    if (cudaMallocFromPoolAsync((void **)&blocks, bytes, pool, st) != cudaSuccess) {
-      cudaGetLastError();  // no room for the blocks: the scalar kernel
+    e = assemble_blocks(a, vals != nullptr, st);
+    if (e == cudaErrorMemoryAllocation) {
       kp = 1;
+      scalar_jac = vals != nullptr;
+    } else if (e != cudaSuccess) {
+      return cuda_fail(e, "assembly launch");
     }
   }
-  if (timing) cudaEventRecord(ev_k0, st);
-  if (kp == 5) {  // writes every entry of R and vals
-    const S2Nodes nd{L.num_nodes, d_ne_ptr, d_ne_list, L.blkmax};
-    e = launch_assemble_2d(a, L.energy != 0, carreau, vals != nullptr, d_s2, L.num_elems, nd,
-                           blocks, num_sms, st);
-    const cudaError_t f = cudaFreeAsync(blocks, st);  // also after a failed launch
-    if (e == cudaSuccess) e = f;
-    if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
-  } else {
+  if (kp != 5) {
     e = cudaMemsetAsync(R, 0, sizeof(double) * L.N, st);
     if (e == cudaSuccess && vals) e = cudaMemsetAsync(vals, 0, sizeof(double) * L.nnz, st);
     if (e != cudaSuccess) return cuda_fail(e, "assembly zeroing");
   }
   if (kp >= 2) tc_grid = 2 * num_sms;
+  auto species = [&](int c) {
+    const int n = L.color_ptr[c + 1] - L.color_ptr[c];
+    return L.dim == 3 && path != 1
+               ? launch_assemble_species_sf(a, L.energy != 0, vals != nullptr, d_sf,
+                                            d_color_elems + L.color_ptr[c], n, num_sms, st)
+               : launch_assemble_species(a, L.dim, L.energy != 0, vals != nullptr,
+                                         d_color_elems + L.color_ptr[c], n, st);
+  };
   for (int c = 0; c < ncol; c++) {
     const int n = L.color_ptr[c + 1] - L.color_ptr[c];
     if (kp == 4)
@@ -357,14 +380,17 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
       e = launch_assemble(a, L.dim, L.energy != 0, carreau, vals != nullptr,
                           d_color_elems + L.color_ptr[c], n, st);
     if (e != cudaSuccess) return cuda_fail(e, "assembly launch");
-    if (L.nspec > 0) {
-      e = L.dim == 3 && path != 1
-              ? launch_assemble_species_sf(a, L.energy != 0, vals != nullptr, d_sf,
-                                           d_color_elems + L.color_ptr[c], n, num_sms, st)
-              : launch_assemble_species(a, L.dim, L.energy != 0, vals != nullptr,
-                                        d_color_elems + L.color_ptr[c], n, st);
-      if (e != cudaSuccess) return cuda_fail(e, "species assembly launch");
-    }
+    if (L.nspec > 0 && !scalar_jac && (e = species(c)) != cudaSuccess)
+      return cuda_fail(e, "species assembly launch");
+  }
+  if (scalar_jac) {
+    AsmArgs r = a;
+    r.status = d_status + 2;  // the elements are counted already
+    e = assemble_blocks(r, false, st);
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation)
+      return cuda_fail(e, "assembly launch");
+    for (int c = 0; c < ncol && L.nspec > 0; c++)
+      if ((e = species(c)) != cudaSuccess) return cuda_fail(e, "species assembly launch");
   }
   if (num_sides > 0) {
     SideArgs sa{num_sides, d_side_elem, d_side_side, d_side_type, d_side_val};
@@ -377,7 +403,7 @@ int Context::assemble(const double *x, double *R, double *vals, cudaStream_t st)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev_k0, ev_k1);
     kernel_ms += ms;
-    kernel_launches += (kp == 5 ? 2 : ncol) + (L.nspec > 0 ? ncol : 0);
+    kernel_launches += (kp == 5 ? 0 : ncol) + (L.nspec > 0 ? ncol : 0);
   }
   return 0;
 }

@@ -57,7 +57,7 @@ struct Context {
   cudaMemPool_t pool = nullptr;
   int num_sms = 0;
   double *d_x = nullptr, *d_R = nullptr, *d_vals = nullptr;
-  int *d_status = nullptr;
+  int *d_status = nullptr;  // bad elements and the first one; [2], [3]: counted elsewhere already
   double *d_elem_rho = nullptr;  // per-element density (gb_set_element_density); NULL: none
   // transient terms of later assemblies: device time derivative (N) and
   // (1 + 2 theta) / delta_t; NULL / 0 when steady
@@ -79,7 +79,8 @@ struct Context {
   int init(const gb_problem_desc *d);
   int set_material(const gb_material &m);
   AsmArgs args(const double *x, double *R, double *vals) const;
-  // zero R (and vals), then launch one kernel per colour on st
+  // R (and vals) on st
+  cudaError_t assemble_blocks(const AsmArgs &a, bool jac, cudaStream_t st);
   int assemble(const double *x, double *R, double *vals, cudaStream_t st);
   int reset_status();
   int check_status();

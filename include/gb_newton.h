@@ -140,7 +140,13 @@ void *gb_stream(gb_ctx *ctx);
  * are summed by factors too unless path 1 is set.  A residual-only
  * assembly uses the same kernel as the full one under paths 0, 1, 3 and 4,
  * so its R is bitwise the full assembly's; under path 2 it uses path 1.  All
- * give the same matrix to rounding. */
+ * give the same matrix to rounding.
+ * The 2-D element blocks take 3,192 bytes an element (6,504 with the energy
+ * equation; 168 and 240 for a residual) of device memory, which the context
+ * keeps for its next assembly and the driver takes back when another
+ * allocation of the process needs it.  Without room for them a Jacobian is
+ * formed by path 1, with R as the residual-only assembly forms it; without
+ * room for the residual's blocks either R comes from path 1 too. */
 int gb_set_assembly_path(gb_ctx *ctx, int path);
 
 /* Node order of the ILU(0) preconditioner of later solves.

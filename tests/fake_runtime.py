@@ -1,5 +1,6 @@
-"""Runs a test's script in a process whose CUDA runtime is fake_cudart.c: the
-library's own host code with calls that can be made to fail, on any machine."""
+"""Runs a test's script in a process with a C file preloaded over the CUDA
+runtime: fake_cudart.c in its place, for the library's host code with calls that
+can be made to fail on any machine, or limit_pool.c on a GPU."""
 import os
 import shutil
 import subprocess
@@ -21,15 +22,15 @@ cavity = lambda nx, ny: pb.lid_cavity_2d(0, mesh=pb.box_mesh(2, nx, ny))
 """
 
 
-def run(script, tmp_path):
+def run(script, tmp_path, source="fake_cudart.c"):
     """The script's output; a failure of the script fails the test."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     inc = os.path.join(os.path.dirname(os.path.realpath(nvcc)), "..", "include")
-    so = os.path.join(str(tmp_path), "fake_cudart.so")
+    so = os.path.join(str(tmp_path), "preloaded.so")
     subprocess.run(["gcc", "-std=c11", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", inc,
-                    os.path.join(ROOT, "tests", "fake_cudart.c"), "-o", so], check=True)
+                    os.path.join(ROOT, "tests", source), "-o", so, "-ldl"], check=True)
     env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=ROOT)
     r = subprocess.run([sys.executable, "-c", PREAMBLE + textwrap.dedent(script)], env=env,
                        cwd=ROOT, capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.returncode == 0, (r.returncode, r.stdout + r.stderr)
     return r.stdout
