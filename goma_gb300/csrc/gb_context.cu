@@ -130,6 +130,13 @@ Context::~Context() {
   if (d_ne_ptr) cudaFree(d_ne_ptr);
   if (d_ne_list) cudaFree(d_ne_list);
   if (pool) cudaMemPoolDestroy(pool);
+  if (graph_blocks) {  // what graphs still hold is of no use without the context
+    {
+      std::lock_guard<std::mutex> lock(graph_blocks->m);
+      for (auto &b : graph_blocks->blocks) b.done = true;
+    }
+    graph_blocks->free_done();
+  }
   if (ev_k0) cudaEventDestroy(ev_k0);
   if (ev_k1) cudaEventDestroy(ev_k1);
   if (stream) cudaStreamDestroy(stream);
@@ -227,6 +234,7 @@ int Context::init(const gb_problem_desc *d) {
       if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return cuda_fail(e, "pool");
       unsigned long long keep = ~0ull;  // kept for the next assembly, freed with the context
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      graph_blocks = std::make_shared<GraphBlocks>();
     }
   }
   if (L.dim == 3) {
@@ -313,20 +321,104 @@ AsmArgs Context::args(const double *x, double *R, double *vals) const {
   return a;
 }
 
+// cudaMalloc and cudaFree while some stream of the process is captured
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+void GraphBlocks::free_done() {
+  std::vector<void *> gone;
+  {
+    std::lock_guard<std::mutex> lock(m);
+    for (size_t i = blocks.size(); i-- > 0;)
+      if (blocks[i].done) {
+        gone.push_back(blocks[i].p);
+        blocks.erase(blocks.begin() + i);
+      }
+    done = 0;
+  }
+  RelaxedCapture relaxed;
+  for (void *p : gone) cudaFree(p);
+}
+
+// Blocks for an assembly that is being captured into graph; NULL: no room.
+double *Context::graph_scratch(size_t bytes, cudaStream_t st, unsigned long long capture,
+                               cudaGraph_t graph) {
+  struct Held {
+    std::shared_ptr<GraphBlocks> of;
+    void *p;
+  };
+  GraphBlocks &G = *graph_blocks;
+  {
+    std::lock_guard<std::mutex> lock(G.m);
+    for (auto &b : G.blocks)
+      if (!b.done && b.capture == capture && b.st == st && b.bytes >= bytes) return (double *)b.p;
+  }
+  RelaxedCapture relaxed;
+  void *p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  auto *held = new Held{graph_blocks, p};
+  cudaUserObject_t obj = nullptr;
+  cudaError_t e = cudaUserObjectCreate(
+      &obj, held,
+      [](void *h) {
+        Held *held = static_cast<Held *>(h);
+        {
+          std::lock_guard<std::mutex> lock(held->of->m);
+          for (auto &b : held->of->blocks)
+            if (b.p == held->p) {
+              b.done = true;
+              held->of->done++;
+            }
+        }
+        delete held;
+      },
+      1, cudaUserObjectNoDestructorSync);
+  if (e == cudaSuccess) {
+    {
+      std::lock_guard<std::mutex> lock(G.m);
+      G.blocks.push_back({p, bytes, capture, st, false});
+    }
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e == cudaSuccess) return (double *)p;
+    cudaUserObjectRelease(obj, 1);  // marks the block
+  } else {
+    delete held;
+    cudaFree(p);
+  }
+  cudaGetLastError();
+  return nullptr;
+}
+
 // Flow rows of a 2-D mesh from element blocks (every entry of R and, with it,
 // vals).  cudaErrorMemoryAllocation: no room for the blocks, nothing done.
 cudaError_t Context::assemble_blocks(const AsmArgs &a, bool jac, cudaStream_t st) {
   const size_t bytes =
       sizeof(double) * s2_scratch_values(L.energy != 0, jac) * (size_t)L.num_elems;
   double *blocks = nullptr;
-  if (cudaMallocFromPoolAsync((void **)&blocks, bytes, pool, st) != cudaSuccess) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(st, &cs, &capture, &graph) != cudaSuccess) cudaGetLastError();
+  const bool captured = cs == cudaStreamCaptureStatusActive;
+  if (captured) {
+    blocks = graph_scratch(bytes, st, capture, graph);
+  } else if (cudaMallocFromPoolAsync((void **)&blocks, bytes, pool, st) != cudaSuccess) {
     cudaGetLastError();
-    return cudaErrorMemoryAllocation;
+    blocks = nullptr;
   }
+  if (!captured && graph_blocks->done > 0) graph_blocks->free_done();
+  if (!blocks) return cudaErrorMemoryAllocation;
   const S2Nodes nd{L.num_nodes, d_ne_ptr, d_ne_list, L.blkmax};
   const cudaError_t e = launch_assemble_2d(a, L.energy != 0, carreau, jac, d_s2, L.num_elems, nd,
                                            blocks, num_sms, st);
-  const cudaError_t f = cudaFreeAsync(blocks, st);  // also after a failed launch
+  // also after a failed launch
+  const cudaError_t f = captured ? cudaSuccess : cudaFreeAsync(blocks, st);
   kernel_launches += timing ? 2 : 0;
   return e != cudaSuccess ? e : f;
 }

@@ -2,20 +2,44 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <memory>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/gb_newton.h"
 #include "gb_device.h"
 #include "gb_layout.h"
 #include "gb_solve.h"
 
-#include <memory>
-
 namespace gb {
 
 extern thread_local std::string g_err;
 int fail(const std::string &m);
 int cuda_fail(cudaError_t e, const char *where);
+
+// Element blocks of captured 2-D assemblies.  They belong to the graph that
+// the assembly was captured into, for as long as it, a copy or an instance of
+// it is there: plain memory, so that the graph holds nothing but kernels and
+// can be instantiated any number of times or become a child graph (allocation
+// and free nodes allow neither).  The graph's end only marks them, since no
+// CUDA call may be made there; the context frees them at its next assembly.
+// The mutex is never held over a CUDA call: the graph's end may come from
+// inside one.
+struct GraphBlocks {
+  struct Block {
+    void *p;
+    size_t bytes;
+    unsigned long long capture;  // assemblies of one capture on one stream follow
+    cudaStream_t st;             // one another and share their blocks
+    bool done;
+  };
+  std::mutex m;
+  std::vector<Block> blocks;
+  std::atomic<int> done{0};
+  void free_done();
+};
 
 struct Context {
   gb_problem_desc desc{};
@@ -51,10 +75,11 @@ struct Context {
   int *d_color_elems = nullptr;
   // 2-D: tables and elements of every node; the pool that the element blocks
   // of an assembly in progress come from (stream-ordered, so that assemblies
-  // on several streams, or captured ones, each have their own)
+  // on several streams each have their own), and those of captured ones
   S2Tables *d_s2 = nullptr;
   int *d_ne_ptr = nullptr, *d_ne_list = nullptr;
   cudaMemPool_t pool = nullptr;
+  std::shared_ptr<GraphBlocks> graph_blocks;
   int num_sms = 0;
   double *d_x = nullptr, *d_R = nullptr, *d_vals = nullptr;
   int *d_status = nullptr;  // bad elements and the first one; [2], [3]: counted elsewhere already
@@ -80,6 +105,8 @@ struct Context {
   int set_material(const gb_material &m);
   AsmArgs args(const double *x, double *R, double *vals) const;
   // R (and vals) on st
+  double *graph_scratch(size_t bytes, cudaStream_t st, unsigned long long capture,
+                        cudaGraph_t graph);
   cudaError_t assemble_blocks(const AsmArgs &a, bool jac, cudaStream_t st);
   int assemble(const double *x, double *R, double *vals, cudaStream_t st);
   int reset_status();

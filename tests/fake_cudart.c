@@ -13,6 +13,8 @@ API int fake_fail_launch = -1;                  /* launches until one fails; < 0
 API long long fake_pool_limit = -1;             /* most bytes of pool allocations; < 0: any */
 API long long fake_pool_live = 0;               /* bytes of them not freed */
 API long long fake_launches = 0;
+API long long fake_malloc_live = 0;             /* cudaMalloc'ed pieces not freed */
+API long long fake_capture = 0;                 /* id of a capture in progress; 0: none */
 API void (*fake_attribute_set)(void) = NULL;    /* called after a kernel's attribute is set */
 
 static cudaError_t last = cudaSuccess;
@@ -71,6 +73,7 @@ API cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, c
 /* ---- memory */
 API cudaError_t cudaMalloc(void **p, size_t n) {
   *p = calloc(n ? n : 1, 1);
+  fake_malloc_live++;
   return *p ? cudaSuccess : done(cudaErrorMemoryAllocation);
 }
 API cudaError_t cudaHostAlloc(void **p, size_t n, unsigned flags) {
@@ -78,6 +81,7 @@ API cudaError_t cudaHostAlloc(void **p, size_t n, unsigned flags) {
   return cudaMalloc(p, n);
 }
 API cudaError_t cudaFree(void *p) {
+  fake_malloc_live -= p != NULL;
   free(p);
   return cudaSuccess;
 }
@@ -137,6 +141,51 @@ API cudaError_t cudaFreeAsync(void *p, cudaStream_t st) {
   fake_pool_live -= (long long)n;
   free((char *)p - 64);
   return cudaSuccess;
+}
+
+/* ---- captures: what the graph holds is let go by fake_graph_gone */
+static struct {
+  cudaHostFn_t f;
+  void *p;
+} held[64];
+static int nheld = 0;
+
+API cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, enum cudaStreamCaptureStatus *st,
+                                         unsigned long long *id, cudaGraph_t *g,
+                                         const cudaGraphNode_t **d, const cudaGraphEdgeData **e,
+                                         size_t *n) {
+  (void)s, (void)d, (void)e, (void)n;
+  *st = fake_capture ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+  if (id) *id = (unsigned long long)fake_capture;
+  if (g) *g = (cudaGraph_t)&held;
+  return cudaSuccess;
+}
+API cudaError_t cudaThreadExchangeStreamCaptureMode(enum cudaStreamCaptureMode *m) {
+  (void)m;
+  return cudaSuccess;
+}
+API cudaError_t cudaUserObjectCreate(cudaUserObject_t *o, void *p, cudaHostFn_t f, unsigned count,
+                                     unsigned flags) {
+  (void)count, (void)flags;
+  held[nheld].f = f;
+  held[nheld].p = p;
+  *o = (cudaUserObject_t)&held[nheld++];
+  return cudaSuccess;
+}
+API cudaError_t cudaGraphRetainUserObject(cudaGraph_t g, cudaUserObject_t o, unsigned count,
+                                          unsigned flags) {
+  (void)g, (void)o, (void)count, (void)flags;
+  return cudaSuccess;
+}
+API cudaError_t cudaUserObjectRelease(cudaUserObject_t o, unsigned count) {
+  (void)o, (void)count;
+  return cudaSuccess;
+}
+API void fake_graph_gone(void) {
+  while (nheld > 0) {
+    nheld--;
+    held[nheld].f(held[nheld].p);
+  }
 }
 
 /* ---- device, streams, events, errors */

@@ -73,3 +73,36 @@ def test_a_failed_launch_gives_the_element_blocks_back(tmp_path):
         assert live.value == 0
         assert fill() == 0 and live.value == 0
     """, tmp_path)
+
+
+def test_blocks_of_captured_assemblies(tmp_path):
+    """They come from the pool no more than they are nodes of the graph: one
+    piece a captured stream, freed at the first assembly after the graph is gone,
+    or with the context, whichever of the two goes first."""
+    fake_runtime.run("""
+    gn = GomaNewton(cavity(5, 4))
+    fill = lambda st=None: gn.matrix_fill_full_device(gn.d_x, gn.d_R, gn.d_vals, st)
+    capture, live, pool = ll("fake_capture"), ll("fake_malloc_live"), ll("fake_pool_live")
+    fill()
+    before = live.value
+    for k in (1, 2):
+        capture.value = k
+        fill()
+        fill()
+        assert live.value == before + 1 and pool.value == 0
+        fill(4096 * k)
+        assert live.value == before + 2
+        capture.value = 0
+        fill()
+        assert live.value == before + 2
+        fake.fake_graph_gone()
+        fill()
+        assert live.value == before and pool.value == 0
+    capture.value = 3
+    fill()
+    capture.value = 0
+    gn.close()
+    assert live.value == 0, live.value
+    fake.fake_graph_gone()
+    assert live.value == 0
+    """, tmp_path)
