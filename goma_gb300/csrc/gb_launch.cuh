@@ -6,6 +6,12 @@
 // kernel before is complete and its writes are visible, so the order of a
 // stream is kept.
 //
+// What an earlier kernel writes is read by ordinary loads: its pointers carry
+// no __restrict__ where the kernel does not write through them, and no __ldg.
+// The read-only path of those asks for data that stay unchanged for the
+// kernel's whole life, which here begins before the earlier kernel's writes
+// are visible.
+//
 // No kernel lets its successor start before its own end
 // (griddepcontrol.launch_dependents): blocks that wait on an SM slowed the
 // sweeps down.  Solves of the 32 x 32 cavity Newton: 229.9 ms without, 215.9

@@ -144,9 +144,9 @@ enum { MLP_FORWARD, MLP_BACK, MLP_GRAD };
 
 template <int OP>
 __global__ void __launch_bounds__(256, 2)
-    mlp_gemm_kernel(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B,
-                    const float *__restrict__ E, float *__restrict__ C, int act, int kchunk,
-                    bool vec_a, bool vec_b, bool vec_c) {
+    mlp_gemm_kernel(int M, int N, int K, const float *A, const float *B, const float *E,
+                    float *__restrict__ C, int act, int kchunk, bool vec_a, bool vec_b,
+                    bool vec_c) {
   dependent_begin();
   constexpr bool AK = OP != MLP_GRAD, BK = OP == MLP_FORWARD;
   union Smem {
@@ -284,9 +284,8 @@ __global__ void __launch_bounds__(256, 2)
 // C[M][N] = A[M][K] W[N][K]^T + bias (tanh): a warp per row, lanes over k
 // (4096 x 1 x 256: 4 us, 10 us as a tile)
 __global__ void __launch_bounds__(256)
-    mlp_forward_narrow_kernel(int M, int N, int K, const float *__restrict__ A,
-                              const float *__restrict__ W, const float *__restrict__ bias,
-                              float *__restrict__ C, int act) {
+    mlp_forward_narrow_kernel(int M, int N, int K, const float *A, const float *W,
+                              const float *bias, float *__restrict__ C, int act) {
   dependent_begin();
   const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m >= M) return;
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(256)
     const float x = a[k];
 #pragma unroll
     for (int j = 0; j < kNarrow; j++)
-      if (j < N) s[j] = fmaf(x, __ldg(W + (int64_t)j * K + k), s[j]);
+      if (j < N) s[j] = fmaf(x, W[(int64_t)j * K + k], s[j]);
   }
 #pragma unroll
   for (int j = 0; j < kNarrow; j++)
@@ -312,8 +311,7 @@ __global__ void __launch_bounds__(256)
 // C[M][K] = (D[M][N] W[N][K]) (1 - H^2), N <= kNarrow: a thread keeps its
 // column of W over its rows
 __global__ void __launch_bounds__(256)
-    mlp_back_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
-                           const float *__restrict__ W, const float *__restrict__ H,
+    mlp_back_narrow_kernel(int M, int N, int K, const float *D, const float *W, const float *H,
                            float *__restrict__ C) {
   dependent_begin();
   for (int k = blockIdx.x * 256 + threadIdx.x; k < K; k += gridDim.x * 256) {
@@ -326,7 +324,7 @@ __global__ void __launch_bounds__(256)
       float s = 0.f;
 #pragma unroll
       for (int j = 0; j < kNarrow; j++)
-        if (j < N) s = fmaf(__ldg(D + (int64_t)m * N + j), w[j], s);
+        if (j < N) s = fmaf(D[(int64_t)m * N + j], w[j], s);
       C[(int64_t)m * K + k] = s * (1.f - h * h);
     }
   }
@@ -337,9 +335,8 @@ __global__ void __launch_bounds__(256)
 // one, four groups of rows a block, 32 rows of the narrow one at a time in
 // shared memory (4096 rows, 256 x 8: 5 us, 21 us as tiles and column sums).
 __global__ void __launch_bounds__(256)
-    mlp_grad_narrow_kernel(int M, int N, int K, const float *__restrict__ D,
-                           const float *__restrict__ X, float *__restrict__ G, int mchunk,
-                           int wide_is_d) {
+    mlp_grad_narrow_kernel(int M, int N, int K, const float *D, const float *X,
+                           float *__restrict__ G, int mchunk, int wide_is_d) {
   dependent_begin();
   constexpr int R = 32;
   __shared__ __align__(16) float q[4][R][kNarrow];
@@ -412,8 +409,7 @@ static void launch_layer(const float *X, int B, int K, int N, const float *W, co
 }
 
 // g[i] = sum over the splits z (in order) of P[z][i]
-__global__ void grad_sum_kernel(int nsplit, int n, const float *__restrict__ P,
-                                float *__restrict__ g) {
+__global__ void grad_sum_kernel(int nsplit, int n, const float *P, float *__restrict__ g) {
   dependent_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -424,7 +420,7 @@ __global__ void grad_sum_kernel(int nsplit, int n, const float *__restrict__ P,
 }
 
 // dY = 2 mask (Y - T) / msum ; per-block partial of sum mask (Y-T)^2
-__global__ void loss_grad_kernel(int n, const float *__restrict__ Y, const float *__restrict__ T,
+__global__ void loss_grad_kernel(int n, const float *Y, const float *__restrict__ T,
                                  const float *__restrict__ mask, float inv_msum,
                                  float *__restrict__ dY, float *__restrict__ part) {
   dependent_begin();
@@ -444,7 +440,7 @@ __global__ void loss_grad_kernel(int n, const float *__restrict__ Y, const float
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__global__ void adam_kernel(int n, float *__restrict__ w, const float *__restrict__ g,
+__global__ void adam_kernel(int n, float *__restrict__ w, const float *g,
                             float *__restrict__ m, float *__restrict__ v, float lr, float b1,
                             float b2, float eps, float c1, float c2) {
   dependent_begin();

@@ -197,8 +197,8 @@ static constexpr int kGsRows = 128;
 static constexpr int kGsBlocks = 8 * 152;  // two waves: 43 us with one at N = 160K
 template <class T, int OP>
 __global__ void __launch_bounds__(256, 4)
-    gs_kernel(int N, int k, const T *__restrict__ V, int64_t ld, const double *__restrict__ h,
-              T *__restrict__ w, double *__restrict__ part) {
+    gs_kernel(int N, int k, const T *__restrict__ V, int64_t ld, const double *h, T *w,
+              double *__restrict__ part) {
   dependent_begin();
   using A = acc_t<T>;
   constexpr int RPT = kGsRows / 32;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256, 4)
 // host[j] the same in page-locked memory, which the host reads after the
 // step: a copy in its place cost 10 us a step, most of it before and after
 __global__ void __launch_bounds__(128)
-    multidot_final_kernel(int nblocks, const double *__restrict__ part, double *__restrict__ out,
+    multidot_final_kernel(int nblocks, const double *part, double *__restrict__ out,
                           double *__restrict__ host) {
   dependent_begin();
   __shared__ double red[4];
@@ -329,7 +329,7 @@ struct SweepIo {
 // norm[0], or with nparts > 0 the root of the sum of part[0..nparts), formed
 // alike by every block and kept in norm[0] and in the host's host[0].
 template <class T, class T2>
-__global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *__restrict__ part,
+__global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *part,
                                   double *norm, double *host, T *y, SweepIo<T2> io) {
   dependent_begin();
   io.start();
@@ -427,7 +427,7 @@ __global__ void to_f32_kernel(int64_t n, const double *__restrict__ x, float *__
     y[i] = (float)x[i];
 }
 
-__global__ void to_f64_kernel(int64_t n, const float *__restrict__ x, double *__restrict__ y) {
+__global__ void to_f64_kernel(int64_t n, const float *x, double *__restrict__ y) {
   dependent_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -451,14 +451,14 @@ __global__ void to_f64_kernel(int64_t n, const float *__restrict__ x, double *__
 template <class T, int LPR, int ROWS>
 __device__ __forceinline__ void spmv_group(int64_t r0, int64_t len, int l,
                                            const int *__restrict__ colidx,
-                                           const T *__restrict__ vals, const T *__restrict__ x,
+                                           const T *__restrict__ vals, const T *x,
                                            acc_t<T> (&s)[4]) {
   using A = acc_t<T>;
   const int *c = colidx + r0;
   const T *v = vals + r0;
 #pragma unroll 4
   for (int64_t k = l; k < len; k += LPR) {
-    const A xv = (A)__ldg(x + c[k]);
+    const A xv = (A)x[c[k]];
 #pragma unroll
     for (int r = 0; r < ROWS; r++) s[r] = fmx((A)v[r * len + k], xv, s[r]);
   }
@@ -468,7 +468,7 @@ template <class T, int LPR>
 __global__ void __launch_bounds__(256)
     spmv_kernel(int ng, const int2 *__restrict__ groups, const int64_t *__restrict__ rowptr,
                 const int *__restrict__ colidx, const T *__restrict__ vals,
-                const T *__restrict__ x, T *__restrict__ y) {
+                const T *x, T *__restrict__ y) {
   dependent_begin();
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPR, l = threadIdx.x % LPR;
   using A = acc_t<T>;
@@ -1453,10 +1453,9 @@ static int gmres(Context *C, const T *b, T *x, double tol, int maxit, int m, int
 static constexpr int kSegRows = 8;  // a tile has at most 8 x 256 unknowns
 template <class T, int OP>
 __global__ void __launch_bounds__(256, 2)
-    seg_gs_kernel(int k, const T *__restrict__ V, int64_t ld, const double *__restrict__ c,
-                  T *__restrict__ w, const int *__restrict__ tseg,
-                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
-                  double *__restrict__ part) {
+    seg_gs_kernel(int k, const T *V, int64_t ld, const double *c, T *w,
+                  const int *__restrict__ tseg, const int64_t *__restrict__ tbeg,
+                  const int64_t *__restrict__ tend, double *__restrict__ part) {
   dependent_begin();
   using A = acc_t<T>;
   __shared__ double red[8][32];
@@ -1519,7 +1518,7 @@ __global__ void __launch_bounds__(256, 2)
 // out[s][j] = sum over the tiles of block s of part[t][j], a warp per (s, j),
 // and the same to the host (multidot_final_kernel)
 __global__ void seg_reduce_kernel(int nseg, int k, const int *__restrict__ tptr,
-                                  const double *__restrict__ part, double *__restrict__ out,
+                                  const double *part, double *__restrict__ out,
                                   double *__restrict__ host) {
   dependent_begin();
   const int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1553,7 +1552,7 @@ __global__ void seg_gemv_kernel(int k, const T *__restrict__ V, int64_t ld,
 // dst = src * alpha[s] on block s; alpha = 1 / sqrt(norm2[s]) for active
 // blocks with a nonzero norm, else 0; and the sweeps' vectors
 template <class T, class T2>
-__global__ void seg_scale_kernel(const T *src, const double *__restrict__ norm2,
+__global__ void seg_scale_kernel(const T *src, const double *norm2,
                                  const int *__restrict__ active, const int *__restrict__ tseg,
                                  const int64_t *__restrict__ tbeg, const int64_t *__restrict__ tend,
                                  T *dst, SweepIo<T2> io) {
