@@ -197,12 +197,15 @@ __global__ void __launch_bounds__(NTH)
       const bool nz = gd > 1.0e-298;
       const double lg = M.lambda * gd;
       // (lg)^a and (1 + lg^a)^((n-1)/a); the other two powers of the model
-      // follow by a division (unless lg^a underflows)
+      // follow by a division (unless lg^a underflows; where it overflows, a
+      // finite number over lg meets the other quotient's zero)
       const double val2 = !nz ? 0.0 : (M.aexp == 2.0 ? lg * lg : pow(lg, M.aexp));
       const double base = 1.0 + val2;
       const double pw = pow(base, (M.nexp - 1.0) / M.aexp);
       mu = M.mu_inf + (M.mu0 - M.mu_inf) * pw;
-      const double val = nz ? (val2 > 1.0e-280 ? val2 / lg : pow(lg, M.aexp - 1.0)) : 0.0;
+      const double val = !nz ? 0.0
+                             : (val2 > 1.0e-280 ? fmin(val2, 1.0e308) / lg
+                                                : pow(lg, M.aexp - 1.0));
       const double dmu = (M.mu0 - M.mu_inf) * (M.nexp - 1.0) * M.lambda * val * (pw / base);
       E.cm[q] = nz ? -dA * (dmu / gd) : 0.0;
       E.gam[0][q] = g00;
