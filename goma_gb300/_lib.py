@@ -121,6 +121,7 @@ def load():
                                                    ip, ctypes.POINTER(ctypes.c_longlong)]),
         "gb_set_triangular_solve": (ctypes.c_int, [vp, ctypes.c_int]),
         "gb_set_sweep_fault": (ctypes.c_int, [vp, ctypes.c_longlong, ctypes.c_int]),
+        "gb_set_factor_fault": (ctypes.c_int, [vp, ctypes.c_longlong, ctypes.c_int]),
         "gb_ilu0_factors": (ctypes.c_int, [vp, dp, ctypes.c_int, dp]),
         "gb_kernel_timing": (ctypes.c_int, [vp, ctypes.c_int, dp, llp]),
         "gb_linear_solve": (ctypes.c_int, [vp, dp, dp, dp, ctypes.POINTER(NewtonOpts), ip, dp]),

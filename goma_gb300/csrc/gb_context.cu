@@ -783,6 +783,13 @@ int gb_set_sweep_fault(gb_ctx *ctx, long long spin_limit, int reverse_lower) {
   return 0;
 }
 
+int gb_set_factor_fault(gb_ctx *ctx, long long spin_limit, int reverse) {
+  if (!ctx) return fail("NULL argument");
+  ctx->c.factor_spin_limit = spin_limit > 0 ? spin_limit : 0;
+  ctx->c.factor_reverse = reverse != 0;
+  return 0;
+}
+
 int gb_set_material(gb_ctx *ctx, const gb_material *mat) {
   if (!ctx || !mat) return fail("NULL argument");
   return ctx->c.set_material(*mat);

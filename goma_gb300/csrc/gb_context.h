@@ -58,6 +58,9 @@ struct Context {
   // host-injected fault of the sync-free sweeps (gb_set_sweep_fault)
   long long sweep_spin_limit = 0;  // polls per wait; <= 0: the default
   int sweep_reverse_lower = 0;
+  // and of the factorisation (gb_set_factor_fault)
+  long long factor_spin_limit = 0;
+  int factor_reverse = 0;
   int ilu_ordering = 0;  // ILU(0) node order: 0 the reference's, 1 multicoloured
   cudaStream_t stream = nullptr;
   double *d_coords = nullptr;

@@ -385,7 +385,7 @@ static cudaError_t launch_ilu(const IluArgs &g, const double *A, T *lu, int sms,
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, sm);
   if (e != cudaSuccess) return e;
-  const int grid = std::min(g.num_nodes, std::max(1, per_sm) * sms);
+  const int grid = g.one_cta ? 1 : std::min(g.num_nodes, std::max(1, per_sm) * sms);
   k<<<grid, NT, sm, st>>>(g, A, lu);
   return cudaGetLastError();
 }

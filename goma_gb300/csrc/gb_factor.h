@@ -24,6 +24,7 @@ struct IluArgs {
   int *done;            // [num_nodes] set when a node's rows are final, then the ticket
   int *error;           // set when a wait gave up
   long long spin_limit; // polls before a wait gives up
+  bool one_cta;         // on a grid of one CTA (an injected fault)
 };
 
 // Shared memory of one CTA for elements of size tsize, and the most there is.

@@ -745,7 +745,7 @@ static IluArgs ilu_args(const Solver *S, const Context *C, int *nfix) {
   g.nbr_off = S->P.nbr_off;
   g.nbr_offT = S->P.nbr_offT;
   g.nbr_self = S->P.nbr_self;
-  g.nodes = S->d_lo_nodes;
+  g.nodes = C->factor_reverse ? S->d_lo_rev : S->d_lo_nodes;
   g.num_nodes = L.num_nodes;
   g.dim = L.dim;
   g.nvn = L.nvn;
@@ -759,7 +759,8 @@ static IluArgs ilu_args(const Solver *S, const Context *C, int *nfix) {
   g.rpiv = S->d_rpiv;
   g.done = S->d_done;
   g.error = (int *)(S->d_flags + 4);
-  g.spin_limit = kSpinLimit;
+  g.spin_limit = C->factor_spin_limit > 0 ? C->factor_spin_limit : kSpinLimit;
+  g.one_cta = C->factor_reverse != 0;
   return g;
 }
 
@@ -1084,6 +1085,16 @@ int Solver::factor(const double *vals, bool fp32, cudaStream_t st) {
     gather_kernel<double><<<1216, 256, 0, st>>>(nnz, d_vmap, vals, d_Ap);
     GB_CU(cudaGetLastError(), "matrix permutation");
     Af = d_Ap;
+  }
+  if (C->factor_reverse && !d_lo_rev) {
+    std::vector<int> rev((size_t)C->L.num_nodes);
+    GB_CU(cudaMemcpy(rev.data(), d_lo_nodes, sizeof(int) * rev.size(), cudaMemcpyDeviceToHost),
+          "reversed nodes");
+    std::reverse(rev.begin(), rev.end());
+    GB_CU(cudaMalloc(&d_lo_rev, sizeof(int) * rev.size()), "reversed nodes");
+    owned.push_back(d_lo_rev);
+    GB_CU(cudaMemcpy(d_lo_rev, rev.data(), sizeof(int) * rev.size(), cudaMemcpyHostToDevice),
+          "reversed nodes");
   }
   const IluArgs g = ilu_args(this, C, nfix);
   GB_CU(cudaMemsetAsync(d_done, 0, sizeof(int) * (size_t)(C->L.num_nodes + 1), st), "ILU flags");

@@ -79,6 +79,7 @@ struct Solver {
   int64_t *d_diag = nullptr;    // position of the diagonal in every row
   int *d_fu = nullptr;          // first unknown per node (shared with C)
   int *d_lo_nodes = nullptr, *d_up_nodes = nullptr;
+  int *d_lo_rev = nullptr;      // the former backwards (gb_set_factor_fault)
   std::vector<int> lo_ptr, up_ptr;
   const double *d_A = nullptr;  // scaled FP64 matrix the factors were built from
   double pivot_tau = 1e-4;      // ILU(0) pivot floor on the row-scaled matrix

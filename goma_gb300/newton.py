@@ -197,6 +197,10 @@ class GomaNewton:
         only end by giving up.  set_sweep_fault() restores the normal sweeps."""
         _lib.check(self._L.gb_set_sweep_fault(self.h, int(spin_limit), 1 if reverse_lower else 0))
 
+    def set_factor_fault(self, spin_limit=0, reverse=False):
+        """The same for the ILU(0) factorisation (gb_set_factor_fault)."""
+        _lib.check(self._L.gb_set_factor_fault(self.h, int(spin_limit), 1 if reverse else 0))
+
     def scale_device(self, d_vals, d_R, d_scale=None):
         """row_sum_scaling_scale on device arrays (in place)."""
         _lib.check(self._L.gb_row_sum_scale_device(self.h, d_vals, d_R, d_scale))

@@ -191,6 +191,12 @@ int gb_set_triangular_solve(gb_ctx *ctx, int mode);
  * context still usable.  (0, 0) restores the normal sweeps.  Applies to
  * the sync-free sweeps only (gb_set_triangular_solve modes 0 and 2). */
 int gb_set_sweep_fault(gb_ctx *ctx, long long spin_limit, int reverse_lower);
+/* The same for the ILU(0) factorisation's waits: with reverse != 0 it hands
+ * its nodes out in reverse order on a grid of one CTA, so that the first wait
+ * runs out, the later ones stop within 1024 polls, and the linear solve (or
+ * gb_ilu0_factors) returns -1 without factors to reuse.  (0, 0) restores the
+ * normal factorisation. */
+int gb_set_factor_fault(gb_ctx *ctx, long long spin_limit, int reverse);
 
 /* Replaces the material of a context (same mesh, DOF map and pattern), as
  * update_parameterC does during continuation (src/ac_conti.c:755,
