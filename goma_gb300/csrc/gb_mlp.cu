@@ -10,8 +10,10 @@
 // live in one flat FP32 buffer (and gradients / Adam moments in three more),
 // so the host can read, write and checksum them in one copy.
 //
-// The products run on the FP32 pipe in FP32 FMA, a sum over k in ascending
-// order: the predictor's accuracy is that of FP32 arithmetic.
+// The products run on the FP32 pipe in FP32 FMA.  A sum over k is split in a
+// fixed way (two groups of k in the tiled kernel, lanes in the narrow ones,
+// parts of the batch for the gradients) and added in a fixed order: results do
+// not depend on timing, and the predictor's accuracy is that of FP32 arithmetic.
 #include <cuda_runtime.h>
 
 #include <algorithm>

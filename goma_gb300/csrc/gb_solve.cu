@@ -4,9 +4,10 @@
 //   SpMV            MV_MSR semantics (src/sl_auxutil.c:373) on the CSR copy
 //   ILU(0)          the preconditioner AztecOO builds for "Preconditioner =
 //                   ilu" (dom_decomp + subdomain ILU(0), src/sl_util.c:556),
-//                   same ordering and pattern; factorised and applied by
-//                   node levels (one warp per node, unknowns of a node in
-//                   order), the level sequence replayed as a CUDA graph
+//                   same ordering and pattern; factorised in one launch
+//                   (gb_factor.cu), applied by sweeps along lines of nodes
+//                   (gb_sweep.cu) or, when asked for, level by level
+//                   (a CTA per node, replayed as a CUDA graph)
 //   GMRES(m)        right-preconditioned restarted GMRES with classical
 //                   Gram-Schmidt + reorthogonalisation (the reference's
 //                   "Solution Algorithm = gmres", Krylov size 30,
@@ -366,11 +367,6 @@ __global__ void scale_copy_kernel(int N, const T *x, int nparts, const double *p
   }
 }
 
-__global__ void axpy_kernel(int N, double a, const double *__restrict__ x, double *__restrict__ y) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
-    y[i] = fma(a, x[i], y[i]);
-}
-
 __global__ void axpy_f32_kernel(int N, double a, const float *__restrict__ x,
                                 double *__restrict__ y) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
@@ -443,8 +439,8 @@ __global__ void to_f64_kernel(int64_t n, const float *x, double *__restrict__ y)
 // that keep a sum, 4 adds instead of 12 for four rows by 8 lanes.  A row's
 // products are added as by 8 lanes of its own.
 //
-// Bound in FP64 by the FP64 pipe (N = 160K, 34 M entries: 58 us of products
-// at 2 a clock and SM) about as much as by HBM (51 us): 82 us, 103 us a row at
+// Bound in FP64 by the FP64 pipe (N = 160K, 38.9 M entries: 62 us of products
+// at 2 a clock and SM) about as much as by HBM (58 us): 82 us, 103 us a row at
 // a time.  Groups are sorted by rows and length: vertex nodes have rows five
 // times as long as centroids, and a warp takes as long as its longest (105 us
 // unsorted), as the launch does, so the longest come first.
@@ -507,7 +503,8 @@ __global__ void __launch_bounds__(256)
 // computed value, NaNs included, differs from it).  Whoever needs a solution
 // value polls the value itself -- no flag, no fence: each is published by one
 // single-copy-atomic store.  A legitimate wait lasts microseconds; the default
-// limit of a wait (kSpinLimit) is ~0.3 s.
+// limit of a wait (kSpinLimit) is 0.9 s of polls through L2 and 0.3 s of polls
+// in shared memory, which warps behind a waiting one make.
 //
 // Row structure used here: a node's unknowns are contiguous and
 // every row of the node holds every own-node column except the energy row,
@@ -910,7 +907,6 @@ int Solver::init(Context *c, int krylov) {
   GB_CU(cudaMalloc(&d_up_nodes, sizeof(int) * S.up_nodes.size()), "sched");
   GB_CU(cudaMemcpy(d_up_nodes, S.up_nodes.data(), sizeof(int) * S.up_nodes.size(),
                    cudaMemcpyHostToDevice), "sched");
-  d_fu = c->d_fu;
   if (L.nvn + L.npres > kMaxNodeDofs) return fail("ILU(0) supports at most 16 unknowns per node");
   maxnb = lmax = blkmax = 0;
   for (int n = 0; n < LP->num_nodes; n++) {

@@ -13,9 +13,9 @@ namespace gb {
 
 struct Context;
 
-// Host-built schedule of the ILU(0) factorisation and triangular solves:
-// nodes grouped by level; all unknowns of one node are handled by one warp
-// in order, so a level only waits for the levels before it.
+// Host-built schedule: nodes grouped by level, each of which depends on the
+// levels before it only.  The order in which the factorisation hands its nodes
+// out, and the launches of the level-scheduled sweeps.
 struct IluSchedule {
   std::vector<int> lo_nodes, lo_ptr;  // forward (L) levels
   std::vector<int> up_nodes, up_ptr;  // backward (U) levels
@@ -77,7 +77,6 @@ struct Solver {
   double *d_line_lo = nullptr, *d_line_up = nullptr;
   float *d_line_lo32 = nullptr, *d_line_up32 = nullptr;
   int64_t *d_diag = nullptr;    // position of the diagonal in every row
-  int *d_fu = nullptr;          // first unknown per node (shared with C)
   int *d_lo_nodes = nullptr, *d_up_nodes = nullptr;
   int *d_lo_rev = nullptr;      // the former backwards (gb_set_factor_fault)
   std::vector<int> lo_ptr, up_ptr;

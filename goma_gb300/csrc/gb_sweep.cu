@@ -21,8 +21,8 @@
 //   far columns   the right-hand side, then the neighbours outside the line's
 //                 last two nodes, oldest first: lane = column, four
 //                 accumulators; each value is polled in L2 until published.
-//                 Loads of factors run ahead of the polls, a batch of kBatch
-//                 chunks of 32 columns at a time.
+//                 The next chunk of 32 columns is on its way while one is
+//                 polled and added.
 //   near columns  the line's two previous nodes: lane = (column, row); their
 //                 values are polled in the shared-memory ring.
 // The warps of a CTA take the tasks of its lines in turn, so while one warp

@@ -47,14 +47,13 @@ struct LineTables {
   // separately); right-hand-side columns hold their index in the node
   std::vector<uint32_t> src;  // offset | energy-row offset << 16
   int64_t num_groups = 0;     // groups of 32 values
-  double mean_line = 0.0;     // nodes per line
   double width = 0.0;         // lines that can be worked on at a time, on average
   bool wide = false;          // some node has more than 8 unknowns
 };
 
 // Tables of the lower (upper = false) or upper sweep of the layout L.
 // Returns -1 when the layout is outside the tables' ranges (a row longer
-// than 65,534 entries, more than 2^32 groups): the node sweeps serve then.
+// than 65,534 entries, more than 2^32 groups): the solver refuses it.
 int build_line_tables(const Layout &L, bool upper, LineTables &T);
 
 struct LineArgs {

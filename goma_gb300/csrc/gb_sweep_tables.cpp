@@ -29,7 +29,6 @@ int build_line_tables(const Layout &L, bool upper, LineTables &T) {
   }
   const int nl = (int)first.size();
   first.push_back(nn);
-  T.mean_line = (double)nn / std::max(1, nl);
   // estimated times and the lines' order.  The lines of the dependencies of a
   // line are before it in node order (after it in the upper sweep), so with
   // key(line) >= the keys of its dependencies a stable sort by key keeps

@@ -182,7 +182,8 @@ int gb_set_triangular_solve(gb_ctx *ctx, int mode);
 
 /* Host-side fault injection for the sync-free sweeps' bounded waits; no
  * counterpart in the reference.  spin_limit sets the polls a wait makes
- * before it gives up (<= 0: the default, 2^22, about 0.3 s).  With
+ * before it gives up (<= 0: the default, 2^22: 0.9 s for a value of another
+ * line, which comes through L2, 0.3 s for one of the same line).  With
  * reverse_lower != 0 the lower sweep hands its lines out in reverse order
  * (every dependency after the line that needs it) on a grid of one CTA,
  * so its first wait can only end by running out: the sweep then finishes
