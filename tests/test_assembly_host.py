@@ -106,3 +106,24 @@ def test_blocks_of_captured_assemblies(tmp_path):
     fake.fake_graph_gone()
     assert live.value == 0
     """, tmp_path)
+
+
+def test_launches_of_an_assembly_are_counted(tmp_path):
+    """bench.py's count: two for the element blocks, one a colour for the scalar
+    kernel, also where it takes over for want of room."""
+    fake_runtime.run("""
+    import bench
+    gn = GomaNewton(cavity(5, 4))
+    count = lambda: bench.assembly_launches(gn, gn.d_x, None)
+    assert count() == 2
+    gn.set_assembly_path(1)
+    assert count() == gn.num_colors == 4
+    gn.set_assembly_path(0)
+    limit = ll("fake_pool_limit")
+    limit.value = 20 * 168
+    assert count() == gn.num_colors + 2
+    limit.value = 0
+    assert count() == gn.num_colors
+    limit.value = -1
+    assert count() == 2
+    """, tmp_path)
