@@ -440,7 +440,8 @@ __global__ void __launch_bounds__(128)
         const int64_t e = nd.ne_list[p] / NN;
         const int k = nd.ne_list[p] % NN;
         if (lane < NV) s += in.R[e * (NV * NN) + k * NV + lane];
-        else if (lane >= nvn) s += in.Rc[e * NP + lane - nvn];
+        // the pressures are the centroid's element's, whoever else has the node
+        else if (lane >= nvn && k == CENT) s += in.Rc[e * NP + lane - nvn];
       }
     A.R[f0 + lane] = s;
   }
@@ -504,8 +505,8 @@ __global__ void __launch_bounds__(128)
     __syncwarp();
     cur = nxt;
   }
-  // Dirichlet rows: 1 per element on the diagonal (species rows get theirs
-  // from the species kernel)
+  // Dirichlet rows: 1 per element on the diagonal, once for a pressure (species
+  // rows get theirs from the species kernel)
   int self = -1;
   if (p1 > p0) self = A.elem_nslot[(int64_t)nd.ne_list[p0] * NN + nd.ne_list[p0] % NN];
   for (int r = 0; r < nr; r++) {
@@ -514,7 +515,8 @@ __global__ void __launch_bounds__(128)
     for (int c = lane; c < rl; c += 32) blk[row(r) + c] = 0.0;
     __syncwarp();
     if (lane == 0 && self >= 0 && (r < NV || r >= nvn))
-      blk[row(r) + (r == Tr ? A.nbr_offT[base + self] : A.nbr_off[base + self]) + r] = p1 - p0;
+      blk[row(r) + (r == Tr ? A.nbr_offT[base + self] : A.nbr_off[base + self]) + r] =
+          r < NV ? p1 - p0 : 1;
   }
   __syncwarp();
   double *out = A.vals + r0;
