@@ -19,7 +19,7 @@ CSRC = os.path.join(ROOT, "goma_gb300", "csrc")
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def library(tmp_path_factory):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     so = os.path.join(tmp_path_factory.mktemp("tables"), "check.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-I",
@@ -32,8 +32,8 @@ def checker(tmp_path_factory):
 
 @pytest.mark.parametrize("ordering", [0, 1], ids=["natural", "multicoloured"])
 @pytest.mark.parametrize("name", list(CASES))
-def test_tables(name, ordering, checker):
+def test_tables(name, ordering, library):
     desc, keep = pb.make_desc(CASES[name][0]())
     msg = ctypes.create_string_buffer(256)
-    assert checker.line_tables_check(ctypes.byref(desc), ordering, msg) == 0, msg.value
+    assert library.line_tables_check(ctypes.byref(desc), ordering, msg) == 0, msg.value
     del keep
